@@ -123,13 +123,11 @@ struct SysParams {
     double Lfix64[3];      // L / 2^64
     // neighbour list
     double rlist2;     // (cutoff + skin)^2, the pair-set test
-    // FP32 prefilter of the pair-set test on fixed-point positions: below
-    // lband_lo a candidate is certainly listed, at or above lband_hi it is
-    // certainly not; in between the exact FP64 test decides
-    float lband_lo, lband_hi;
-    // the same screen in a cell-local FP32 frame (coordinates relative to
-    // the first atom of the home cell); usable when every box edge exceeds
-    // 2 (cutoff + skin + 2 cell diagonals), so no fold is needed
+    // FP32 screen of the pair-set test, in the frame of the home cell's first
+    // atom: below fband_lo a candidate is certainly listed, at or above
+    // fband_hi it is certainly not; in between the exact FP64 test decides.
+    // lframe_ok: every box edge exceeds 2 (cutoff + skin + 2 cell diagonals),
+    // so differences in that frame need no minimum image
     int lframe_ok;
     float fband_lo, fband_hi;
     double skin_half2; // (skin/2)^2
@@ -247,7 +245,9 @@ struct SysParams {
     // the LJ parameters and the largest charge product (0 in FP64)
     double force_r2_safe;
     double4* fp4;    // PME reciprocal forces of this step (sorted; PME systems)
-    int *perm, *rank, *cell_of, *slot, *cell_count, *cell_start, *cellS;
+    int *perm, *rank, *cell_of, *slot, *cell_count, *cell_start;
+    int* cell_sums; // atoms per kScanChunk cells
+    int2* perm0;    // {atom, fixed-point z} by cell, in arrival order (k_cell_scatter)
     int *nbr, *nnbr;
     // PME buffers
     unsigned long long* grid_fix;

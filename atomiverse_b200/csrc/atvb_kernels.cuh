@@ -12,7 +12,8 @@ constexpr int kChunk = 256;     // atoms per item of the per-atom kernels
 constexpr int kRebuildKernels = 6; // launches of one list build (cell sort + rows)
 constexpr long long kCondMinAtoms = 100000; // engines from this size skip them by
                                             // conditional graph nodes
-constexpr int kListChunk = 8;   // cells per item of the list build (warp/cell)
+constexpr int kListChunk = 4;   // warp tasks per item of the list build
+constexpr int kScanChunk = 2048; // cells per item of the cell scan
 constexpr int kGridChunk = 4096; // grid points per item of the PME grid kernels
 constexpr int kLaneClasses = 6;  // pair lanes per atom: 1, 2, 4, 8, 16, 32
 constexpr int kGenLanes = 8;      // lanes per atom of k_pair_general
@@ -47,14 +48,15 @@ struct FftCfg {
 struct LaunchCfg {
     const SysParams* sp = nullptr; // device table of every system
     ItemList atoms;     // kChunk atoms per item (original or sorted order)
-    ItemList list;      // kListChunk cells per item
+    ItemList list;      // kListChunk warp tasks (cells x 2^list_split_log2) per item
+    int list_split_log2 = 0; // warps per cell of the list build (list_split)
     // pair work by [precision][log2 lanes]: each system has its own lane
     // count, chosen from that system alone, so its forces and energies do
     // not depend on which other systems share the engine
     ItemList pair[2][kLaneClasses];
     ItemList pair_gen[2]; // [precision]: systems with types or special pairs
                           // (kChunk / kGenLanes atoms per item)
-    ItemList cells;     // kChunk cells per item
+    ItemList scan;      // kScanChunk cells per item
     ItemList pme_atoms; // kChunk atoms of PME systems
     ItemList pme_grid;  // kGridChunk half-complex grid points per item
     ItemList pme_real;  // kGridChunk real grid points per item

@@ -35,31 +35,32 @@ __host__ __device__ inline void apply_box(SysParams& P, const double L[3], bool 
         P.Lfix64[k] = L[k] / 18446744073709551616.0;
         P.cs_inv[k] = (double)P.nc[k] / L[k];
     }
-    // |r2_fp32 - r2_exact| of the list screen <= 5.4e-7 r2 (three FP32
-    // roundings of each difference, three of the sum) + 3.6 r q (fixed-point
-    // quantum q = L / 2^32 on both atoms); the band doubles both terms
-    const double q = fmax(L[0], fmax(L[1], L[2])) / 4294967296.0;
-    const double band = 2e-6 * P.rlist2 + 8.0 * P.rlist * q + 1e-12;
-    P.lband_lo = nextafterf((float)(P.rlist2 - band), 0.0f);
-    P.lband_hi = nextafterf((float)(P.rlist2 + band), 3.0e38f);
-    // cell-local frame: coordinates up to R = rlist + 2 cell diagonals from
-    // the origin, each carrying <= 3 FP32 roundings (2^-24 R) plus the
-    // fixed-point quantum; the difference one more rounding
+    // |r2_fp32 - r2_exact| of the list screen: coordinates relative to the
+    // first atom of the home cell, up to R from it, each carrying <= 3 FP32
+    // roundings (u R, u = 2^-24) plus the fixed-point quantum q = L / 2^32;
+    // the difference one more rounding.  A candidate of the band lies within
+    // R = rlist + 2 cell diagonals of that atom when no minimum image is
+    // taken; with it R = L / 2, differences reach L (rounding u L), and
+    // L - |d| adds the rounding of L and its own (1.5 u L).  The band doubles
+    // the sum.
+    const double Lmax = fmax(L[0], fmax(L[1], L[2]));
+    const double q = Lmax / 4294967296.0;
     double cs[3];
     for (int k = 0; k < 3; ++k)
         cs[k] = L[k] / (double)P.nc[k];
     const double cdiag = sqrt(cs[0] * cs[0] + cs[1] * cs[1] + cs[2] * cs[2]);
-    const double R = P.rlist + 2.0 * cdiag;
+    const double Rc = P.rlist + 2.0 * cdiag;
+    P.lframe_ok = 1;
+    for (int k = 0; k < 3; ++k)
+        if (!(0.5 * L[k] > Rc + 1e-9))
+            P.lframe_ok = 0;
+    const double R = P.lframe_ok ? Rc : 0.5 * Lmax;
     const double u = 1.0 / 16777216.0;
     const double ec = 3.0 * u * R + 2.0 * q;
-    const double ed = 2.0 * ec + u * P.rlist;
+    const double ed = 2.0 * ec + (P.lframe_ok ? u * P.rlist : 2.5 * u * Lmax);
     const double fband = 2.0 * (2.0 * sqrt(3.0) * P.rlist * ed + 3.0 * u * P.rlist2) + 1e-12;
     P.fband_lo = nextafterf((float)(P.rlist2 - fband), 0.0f);
     P.fband_hi = nextafterf((float)(P.rlist2 + fband), 3.0e38f);
-    P.lframe_ok = 1;
-    for (int k = 0; k < 3; ++k)
-        if (!(0.5 * L[k] > R + 1e-9))
-            P.lframe_ok = 0;
     // mixed pair kernel: bands around the LJ and Coulomb cutoffs (the LJ one
     // stays off where the settling was switched off)
     if (P.mix_band_lj > 0.0)

@@ -142,15 +142,21 @@ Geometry make_geometry(const atvb_system_desc& d, double shrink) {
     // half-reach bins, cell_list.cpp:112-121, reach :186-191) gives the
     // fewest candidates per atom, but the list kernel spends a warp per bin
     // and resolves the stencil per bin, so bins must hold enough atoms to
-    // amortise that: reach 3 from 5 atoms per bin, else reach 2 from 1.5,
-    // else reach 1 (measured: the 262k-ion melt builds fastest at reach 2,
-    // 12 ions per bin; reduced-unit LJ at reach 2, 2.3 atoms per bin).
+    // amortise that: reach 3 from 4 atoms per bin, else reach 2 from 2, else
+    // reach 1; and bins that hold fewer than 5.5 at reach 2 are twice as long
+    // in z (reach 1 there), the axis along which a column's atoms are one run
+    // in z order.  Cell sort and build per step, 256,000 LJ atoms, one build
+    // in ten, by atoms per reach-2 bin (bins at reach 1 / long 2 / 2 / 3):
+    //   1.3: 48 / 61 / 83 / 175 us     2.3: 57 / 57 / 69 / 138 us
+    //   3.8: 66 / 59 / 65 / 115 us     5.8: 91 / 73 / 72 / 104 us
+    //   8.4: 114 / 91 / 83 / 100 us   15.7: 192 / 147 / 119 / 108 us
     // The pair set does not depend on the bins.
     const double density = d.n_atoms / (Lp[0] * Lp[1] * Lp[2]);
     auto per_bin = [&](double reach) { return density * std::pow(g.rlist / reach, 3.0); };
-    const double reach_t = per_bin(3.0) >= 5.0 ? 3.0 : (per_bin(2.0) >= 1.5 ? 2.0 : 1.0);
+    const double reach_t = per_bin(3.0) >= 4.0 ? 3.0 : (per_bin(2.0) >= 2.0 ? 2.0 : 1.0);
     for (int k = 0; k < 3; ++k) {
-        int c = (int)std::floor(Lp[k] / (g.rlist / reach_t));
+        const double reach_k = k == 2 && reach_t == 2.0 && per_bin(2.0) < 5.5 ? 1.0 : reach_t;
+        int c = (int)std::floor(Lp[k] / (g.rlist / reach_k));
         g.nc[k] = c < 1 ? 1 : c;
         g.cs[k] = Lp[k] / g.nc[k];
         int r = (int)std::ceil(g.rlist / g.cs[k] - 1e-12);
@@ -318,6 +324,7 @@ void Slot::replan_cells(double shrink) {
     geo = make_geometry(desc, shrink);
     free_alloc(hp.cell_count);
     free_alloc(hp.cell_start);
+    free_alloc(hp.cell_sums);
     free_alloc(hp.cols);
     for (int k = 0; k < 3; ++k) {
         hp.nc[k] = geo.nc[k];
@@ -328,6 +335,7 @@ void Slot::replan_cells(double shrink) {
     hp.ncol = (int)geo.cols.size();
     hp.cell_count = (int*)dalloc(sizeof(int) * hp.ncell);
     hp.cell_start = (int*)dalloc(sizeof(int) * (hp.ncell + 1));
+    hp.cell_sums = (int*)dalloc(sizeof(int) * ((hp.ncell + kScanChunk - 1) / kScanChunk));
     CK(cudaMemsetAsync(hp.cell_count, 0, sizeof(int) * hp.ncell, stream));
     hp.cols = (int4*)dalloc(sizeof(int4) * geo.cols.size());
     CK(cudaMemcpyAsync(hp.cols, geo.cols.data(), sizeof(int4) * geo.cols.size(),
@@ -514,10 +522,11 @@ Slot::Slot(const atvb_system_desc& d, const DevMem& mem) : desc(d), mem_(mem) {
     hp.rank = di(n);
     hp.cell_of = di(n);
     hp.slot = di(n);
-    hp.cellS = di(n);
+    hp.perm0 = (int2*)dalloc((size_t)n * sizeof(int2));
     hp.nnbr = di(n);
     hp.cell_count = di(hp.ncell);
     hp.cell_start = di(hp.ncell + 1);
+    hp.cell_sums = di((hp.ncell + kScanChunk - 1) / kScanChunk);
     CK(cudaMemsetAsync(hp.cell_count, 0, sizeof(int) * hp.ncell, stream));
     hp.cols = (int4*)dalloc(sizeof(int4) * geo.cols.size());
     CK(cudaMemcpyAsync(hp.cols, geo.cols.data(), sizeof(int4) * geo.cols.size(),
@@ -835,6 +844,18 @@ int Engine::lanes_for(const Slot& sl) const {
     return std::max(1, std::min(G, gmax));
 }
 
+// Warps per cell of the list build (log2), for a launch of `cells` cells
+// holding `atoms` atoms: more than one while the cells alone leave the GPU's
+// warp slots empty and a warp keeps at least two atoms.  A 1,728-ion melt
+// (125 cells of 14 ions): cell sort and build 30 us per step with 8 warps per
+// cell (one build in ten steps, launches included), 57 us with 1.
+static int list_split(long long cells, long long atoms, int num_sms) {
+    int k = 0;
+    while (k < 3 && (cells << k) < (long long)num_sms * 48 && atoms >= (cells << (k + 2)))
+        ++k;
+    return k;
+}
+
 static int lane_class(int G) {
     int k = 0;
     while ((1 << k) < G)
@@ -847,7 +868,7 @@ void Engine::build_lists() {
     for (void* p : list_allocs_)
         mem_.free(p);
     list_allocs_.clear();
-    std::vector<Item> atoms, list, cells, patoms;
+    std::vector<Item> atoms, list, scan, patoms;
     std::vector<int> sys;
     std::vector<Item> pair_by[2][kLaneClasses];
     std::vector<Item> pair_gen[2];
@@ -855,6 +876,14 @@ void Engine::build_lists() {
     int largest = -1;
     pme_slots_.clear();
     int pme_prec = -1, pme_order = -1;
+    long long all_cells = 0, all_atoms = 0;
+    for (const auto& sp : slots_)
+        if (sp && sp->uploaded) {
+            all_cells += sp->hp.ncell;
+            all_atoms += sp->hp.n;
+        }
+    const int split = list_split(all_cells, all_atoms, num_sms_);
+    lc_.list_split_log2 = split;
     for (const auto& sp : slots_) {
         if (!sp || !sp->uploaded)
             continue;
@@ -863,8 +892,8 @@ void Engine::build_lists() {
         sys.push_back(k);
         for (int b = 0; b < P.n; b += kChunk)
             atoms.push_back({k, b});
-        for (int b = 0; b < P.ncell; b += kListChunk)
-            list.push_back({k, b});
+        for (long long b = 0; b < (long long)P.ncell << split; b += kListChunk)
+            list.push_back({k, (int)b});
         sp->lanes = lanes_for(*sp);
         if (P.n > largest) {
             largest = P.n;
@@ -879,8 +908,8 @@ void Engine::build_lists() {
             for (int b = 0; b < P.n; b += kPairBlock / sp->lanes)
                 pv.push_back({k, b});
         }
-        for (int b = 0; b < P.ncell; b += kChunk)
-            cells.push_back({k, b});
+        for (int b = 0; b < P.ncell; b += kScanChunk)
+            scan.push_back({k, b});
         if (P.prec == kMixed)
             lc_.any_mixed = 1;
         else
@@ -912,7 +941,7 @@ void Engine::build_lists() {
             lc_.pair[p][c] = make_list(list_allocs_, pair_by[p][c], num_sms_ * 16, mem_);
     for (int p = 0; p < 2; ++p)
         lc_.pair_gen[p] = make_list(list_allocs_, pair_gen[p], num_sms_ * 16, mem_);
-    lc_.cells = make_list(list_allocs_, cells, g_light, mem_);
+    lc_.scan = make_list(list_allocs_, scan, g_light, mem_);
     lc_.pme_atoms = make_list(list_allocs_, patoms, g_light, mem_);
     lc_.nsys = (int)sys.size();
     if (!sys.empty()) {
@@ -1595,13 +1624,14 @@ LaunchCfg Engine::restricted_cfg(int id) {
         return it->second.second;
     Slot* s = slot(id);
     const SysParams& P = s->hp;
-    std::vector<Item> atoms, list, cells, pair, patoms;
+    std::vector<Item> atoms, list, scan, pair, patoms;
     for (int b = 0; b < P.n; b += kChunk)
         atoms.push_back({id, b});
-    for (int b = 0; b < P.ncell; b += kListChunk)
-        list.push_back({id, b});
-    for (int b = 0; b < P.ncell; b += kChunk)
-        cells.push_back({id, b});
+    const int split = list_split(P.ncell, P.n, num_sms_);
+    for (long long b = 0; b < (long long)P.ncell << split; b += kListChunk)
+        list.push_back({id, (int)b});
+    for (int b = 0; b < P.ncell; b += kScanChunk)
+        scan.push_back({id, b});
     const int pchunk = kPairBlock / (P.general ? kGenLanes : s->lanes);
     for (int b = 0; b < P.n; b += pchunk)
         pair.push_back({id, b});
@@ -1612,7 +1642,8 @@ LaunchCfg Engine::restricted_cfg(int id) {
     c.sp = d_sp_;
     c.atoms = make_list(list_allocs_, atoms, num_sms_ * 16, mem_);
     c.list = make_list(list_allocs_, list, num_sms_ * 32, mem_);
-    c.cells = make_list(list_allocs_, cells, num_sms_ * 16, mem_);
+    c.list_split_log2 = split;
+    c.scan = make_list(list_allocs_, scan, num_sms_ * 16, mem_);
     for (int p = 0; p < 2; ++p) {
         for (int k = 0; k < kLaneClasses; ++k)
             c.pair[p][k] = ItemList{};

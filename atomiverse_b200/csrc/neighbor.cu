@@ -40,21 +40,62 @@ __global__ void k_cell_count(const Item* items, int nitems,
     }
 }
 
-// Stage 2: exclusive scan of the cell counts, one block per system.
-__global__ void k_cell_scan(const int* sys_list, const SysParams* sp) {
-    const SysParams& P = sp[sys_list[blockIdx.x]];
-    if (!P.st->rebuild)
-        return;
-    __shared__ int warp_tot[32];
-    __shared__ int carry;
-    if (threadIdx.x == 0)
-        carry = 0;
-    __syncthreads();
+// Stages 2 and 3: exclusive scan of the cell counts over chunks of kScanChunk
+// cells: the chunk sums, then every chunk's block adds up the sums before its
+// own and scans its cells.  One block per system took 440 us at 1,000,188 LJ
+// atoms (430k cells walked by 1,024 threads); the two launches take 15 us.
+__global__ void __launch_bounds__(kChunk)
+    k_cell_sums(const Item* items, int nitems, const SysParams* sp) {
+    __shared__ int tot[kChunk / 32];
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const Item item = items[it];
+        const SysParams& P = sp[item.sys];
+        if (!P.st->rebuild)
+            continue;
+        const int* __restrict__ count = P.cell_count;
+        int v = 0;
+#pragma unroll
+        for (int k = 0; k < kScanChunk / kChunk; ++k) {
+            const int c = item.begin + k * kChunk + threadIdx.x;
+            v += c < P.ncell ? count[c] : 0;
+        }
+        v = __reduce_add_sync(0xffffffffu, v);
+        if ((threadIdx.x & 31) == 0)
+            tot[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int w = 0; w < kChunk / 32; ++w)
+                t += tot[w];
+            P.cell_sums[item.begin / kScanChunk] = t;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kChunk)
+    k_cell_scan(const Item* items, int nitems, const SysParams* sp) {
+    constexpr int kPer = kScanChunk / kChunk;
+    __shared__ int tot[kChunk / 32], pre[kChunk / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int base = 0; base < P.ncell; base += blockDim.x) {
-        const int c = base + threadIdx.x;
-        const int v = c < P.ncell ? P.cell_count[c] : 0;
-        int incl = v;
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const Item item = items[it];
+        const SysParams& P = sp[item.sys];
+        if (!P.st->rebuild)
+            continue;
+        const int ncell = P.ncell, chunk = item.begin / kScanChunk;
+        int before = 0;
+        for (int k = threadIdx.x; k < chunk; k += kChunk)
+            before += P.cell_sums[k];
+        before = __reduce_add_sync(0xffffffffu, before);
+        const int c0 = item.begin + threadIdx.x * kPer;
+        int v[kPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            v[k] = c0 + k < ncell ? P.cell_count[c0 + k] : 0;
+            sum += v[k];
+        }
+        int incl = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -62,36 +103,30 @@ __global__ void k_cell_scan(const int* sys_list, const SysParams* sp) {
                 incl += t;
         }
         if (lane == 31)
-            warp_tot[w] = incl;
+            tot[w] = incl;
+        if (lane == 0)
+            pre[w] = before;
         __syncthreads();
-        if (w == 0) {
-            const int nw = blockDim.x >> 5;
-            int t = lane < nw ? warp_tot[lane] : 0;
+        int base = incl - sum;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, t, o);
-                if (lane >= o)
-                    t += u;
+        for (int k = 0; k < kChunk / 32; ++k)
+            base += pre[k] + (k < w ? tot[k] : 0);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (c0 + k < ncell) {
+                P.cell_start[c0 + k] = base;
+                P.cell_count[c0 + k] = 0; // ready for the next rebuild
             }
-            if (lane < nw)
-                warp_tot[lane] = t; // inclusive over warps
+            base += v[k];
         }
-        __syncthreads();
-        const int before = (w > 0 ? warp_tot[w - 1] : 0) + carry;
-        if (c < P.ncell) {
-            P.cell_start[c] = before + incl - v;
-            P.cell_count[c] = 0; // ready for the next rebuild
-        }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1)
-            carry = before + incl;
+        if (item.begin == 0 && threadIdx.x == 0)
+            P.cell_start[ncell] = P.n;
         __syncthreads();
     }
-    if (threadIdx.x == 0)
-        P.cell_start[P.ncell] = carry;
 }
 
-// Stage 3: scatter atom ids into their cells.
+// Stage 4: scatter atom ids and the fixed-point z that orders them into
+// their cells, in arrival order.
 __global__ void k_cell_scatter(const Item* items, int nitems,
                                const SysParams* sp) {
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
@@ -102,49 +137,42 @@ __global__ void k_cell_scatter(const Item* items, int nitems,
         const int i = item.begin + threadIdx.x;
         if (i >= P.n)
             continue;
-        P.perm[P.cell_start[P.cell_of[i]] + P.slot[i]] = i;
+        P.perm0[P.cell_start[P.cell_of[i]] + P.slot[i]] =
+            make_int2(i, (int)pos_fix(P.z[i], P.fix_scale[2]));
     }
 }
 
-// Stage 4: order each cell by original index, so the permutation (and with
-// it every later summation order) is independent of atomic arrival order.
-__global__ void k_cell_sort(const Item* citems, int nitems,
-                            const SysParams* sp) {
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-        const Item item = citems[it];
-        const SysParams& P = sp[item.sys];
-        if (!P.st->rebuild)
-            continue;
-        const int c = item.begin + threadIdx.x;
-        if (c >= P.ncell)
-            continue;
-        const int a = P.cell_start[c], b = P.cell_start[c + 1];
-        for (int k = a + 1; k < b; ++k) {
-            const int v = P.perm[k];
-            int m = k - 1;
-            while (m >= a && P.perm[m] > v) {
-                P.perm[m + 1] = P.perm[m];
-                --m;
-            }
-            P.perm[m + 1] = v;
-        }
-    }
-}
-
-// Stage 5: inverse permutation, sorted positions, reference positions.
+// Stage 5: order each cell by z, ties by original index, so the permutation
+// (and with it every later summation order) is independent of atomic arrival
+// order.  An atom's place in its cell is the number of the cell's atoms
+// before it (independent loads; an insertion sort per cell, a serial chain
+// through memory, took 39 us for the 13 atoms per cell of a 1,728-ion melt).
+// Cells of a column are consecutive, so a column is one run of atoms in z
+// order, and the atoms of it that a sphere cuts out lie close together: the
+// pair kernel's gathers then touch fewer lines.  The sorted records, the
+// permutation and the reference positions are written here too.
 __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
         if (!P.st->rebuild)
             continue;
-        const int s = item.begin + threadIdx.x;
-        if (s >= P.n)
+        const int t = item.begin + threadIdx.x;
+        if (t >= P.n)
             continue;
-        const int i = P.perm[s];
-        P.rank[i] = s;
-        P.cellS[s] = P.cell_of[i];
+        const int2* __restrict__ perm0 = P.perm0;
+        const int2 me = perm0[t];
+        const int i = me.x;
         const double x = P.x[i], y = P.y[i], z = P.z[i], q = P.q[i];
+        const int c = P.cell_of[i];
+        const int a = P.cell_start[c], b = P.cell_start[c + 1];
+        int s = a;
+        for (int k = a; k < b; ++k) {
+            const int2 o = perm0[k];
+            s += (unsigned)o.y < (unsigned)me.y || (o.y == me.y && o.x < i) ? 1 : 0;
+        }
+        P.perm[s] = i;
+        P.rank[i] = s;
         P.posd4[s] = make_double4(x, y, z, q);
         int4 v;
         v.x = (int)pos_fix(x, P.fix_scale[0]);
@@ -240,230 +268,295 @@ ATVB_DEV unsigned special_class(const SysParams& P, int i, int j) {
     return 0u;
 }
 
-// Stage 6 (items of kListChunk cells): one warp per cell.  Every atom of a
-// cell has the same stencil, so the warp resolves the stencil columns once
-// (up to 32 at a time, one per lane, into runs of sorted atoms laid end to
-// end by a warp prefix sum), loads each window of 32 consecutive candidates
-// once, and tests that window against every atom of the cell in turn,
-// appending hits to that atom's row with a ballot.  Rows list candidates in
-// column order.  Candidates are screened in FP32 on the fixed-point
-// positions (16 bytes per candidate, exact integer minimum image); only
-// those whose FP32 distance lies within the error band of
-// r^2 = (cutoff + skin)^2 take the exact FP64 test, so the listed set is
-// exactly the FP64 one.
-constexpr int kCellAtomsWarp = 32; // atoms of one cell handled per pass
+// Stage 6 (items of kListChunk warp tasks): 2^split_log2 warps per cell, each
+// for its share of the cell's atoms (one warp per cell once the cells alone
+// fill the GPU; the rows do not depend on the split).  Every atom of a cell
+// has the same stencil, so the warp resolves the stencil columns once (up to
+// 32 at a time, one per lane, into runs of sorted atoms laid end to end by a
+// warp prefix sum), loads each window of 32 consecutive candidates once, and
+// tests it against kListAtoms atoms of the cell, appending hits to each
+// atom's row with a ballot.  Rows list candidates in column order.
+//
+// The test is FP32, in the frame of the cell's first atom (exact 32-bit
+// fixed-point differences, rounded to FP32 once); FOLD adds the minimum
+// image of the difference, for boxes where two such coordinates can lie
+// further apart than half an edge.  Its error is bounded (apply_box): below
+// fband_lo a candidate is certainly listed, at or above fband_hi certainly
+// not.  A candidate in between is appended, and a row that got one is
+// settled once it is complete (settle_row) by the exact FP64 test, so the
+// listed set is exactly the FP64 one.
+//
+// Bound by instruction issue (63 % of the issue slots at 24 warps per SM).
+// What a window costs before its first atom (finding each lane's column,
+// loading and converting the candidate) is shared by the atoms of the cell;
+// candidates of the error band are settled per row, not per window, so the
+// window loop has no rare path.  At 8 atoms per pass and 24 warps, cell sort
+// and build per step with one build in nine: 1,000,188 LJ atoms 332 -> 147
+// us, the 262,144-ion melt 184 -> 141 us, 24 LJ replicas of 256 to 32,768
+// atoms 90 -> 68 us (16 warps: 175 / 171 / 72; 4 atoms per pass: 162 / 163 / 72).
+constexpr int kListAtoms = 8;
+constexpr int kListWarps = kListChunk;
+constexpr int kListBlocks = 6; // per SM: 24 warps of 80 registers
 
-__global__ void __launch_bounds__(256)
-    k_build_list(const Item* items, int nitems, const SysParams* sp) {
-    const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    __shared__ int4 sq[8][kCellAtomsWarp];
-    __shared__ float4 sr[8][kCellAtomsWarp];
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-        const Item item = items[it];
-        const SysParams& P = sp[item.sys];
-        if (!P.st->rebuild)
-            continue;
-        const int c = item.begin + warp;
-        if (c >= P.ncell)
-            continue; // warp-uniform
-        // every field the loops use, read once: the row stores below could
-        // alias SysParams as far as the compiler knows, and would force a
-        // reload of any field read after them
-        const int nc0 = P.nc[0], nc1 = P.nc[1], nc2 = P.nc[2];
-        int* __restrict__ nbr = P.nbr;
-        const bool has_sp = P.has_special != 0;
-        const double L[3] = {P.L[0], P.L[1], P.L[2]};
-        const double hL[3] = {P.halfL[0], P.halfL[1], P.halfL[2]};
-        const double rl2 = P.rlist2;
-        const int cap = P.cap, ncol = P.ncol;
-        const int4* __restrict__ cols = P.cols;
-        const int* __restrict__ cstart = P.cell_start;
-        const double4* __restrict__ pos = P.posd4;
-        const int4* __restrict__ lp = P.lpos;
-        const float sx = P.Lf_fix[0], sy = P.Lf_fix[1], sz = P.Lf_fix[2];
-        const float blo = P.lband_lo, bhi = P.lband_hi;
-        const float flo = P.fband_lo, fhi = P.fband_hi;
-        const bool local = P.lframe_ok != 0;
-        const int cz = c % nc2, cy = (c / nc2) % nc1, cx = c / (nc1 * nc2);
-        const int cs = cstart[c], ce = cstart[c + 1];
-        for (int i0 = cs; i0 < ce; i0 += kCellAtomsWarp) {
-            const int ni = min(kCellAtomsWarp, ce - i0);
-            const int4 org = lp[i0];
-            __syncwarp();
-            if (lane < ni) {
-                const int4 q = lp[i0 + lane];
-                sq[warp][lane] = q;
-                sr[warp][lane] = make_float4((float)(int)((unsigned)q.x - (unsigned)org.x) * sx,
-                                             (float)(int)((unsigned)q.y - (unsigned)org.y) * sy,
-                                             (float)(int)((unsigned)q.z - (unsigned)org.z) * sz,
-                                             0.0f);
-            }
-            __syncwarp();
-            int cnt = 0; // row length of atom i0 + lane
-            for (int c0 = 0; c0 < ncol; c0 += 32) {
+// FP32 squared distance of two points of the cell's frame.
+template <bool FOLD>
+ATVB_DEV float frame_r2(float Lx, float Ly, float Lz, float ax, float ay, float az, float rx,
+                        float ry, float rz) {
+    float dx = ax - rx, dy = ay - ry, dz = az - rz;
+    if (FOLD) {
+        dx = fminf(fabsf(dx), Lx - fabsf(dx));
+        dy = fminf(fabsf(dy), Ly - fabsf(dy));
+        dz = fminf(fabsf(dz), Lz - fabsf(dz));
+    }
+    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+// A point of the frame whose origin is `org`.
+ATVB_DEV float3 frame_pos(const SysParams& P, int4 q, int4 org) {
+    return make_float3((float)(int)((unsigned)q.x - (unsigned)org.x) * P.Lf_fix[0],
+                       (float)(int)((unsigned)q.y - (unsigned)org.y) * P.Lf_fix[1],
+                       (float)(int)((unsigned)q.z - (unsigned)org.z) * P.Lf_fix[2]);
+}
+
+// The entries of atom i's row (cnt of them, those below the capacity stored)
+// whose FP32 distance is in the error band, decided by the exact FP64 test:
+// the row is compacted in place, in order.  About one row in a thousand.
+// Returns the new length.  (A row cut at its capacity keeps the entries it
+// has; it is reported and rebuilt.)
+__device__ __noinline__ int settle_row(const SysParams& P, int i, int org_i, int cnt) {
+    const int lane = threadIdx.x & 31;
+    int* row = P.nbr + (size_t)i * P.cap;
+    const int stored = min(cnt, P.cap);
+    const double L[3] = {P.L[0], P.L[1], P.L[2]};
+    const double hL[3] = {P.halfL[0], P.halfL[1], P.halfL[2]};
+    const float Lx = (float)L[0], Ly = (float)L[1], Lz = (float)L[2];
+    const double rl2 = P.rlist2;
+    const bool fold = !P.lframe_ok;
+    const int4 org = P.lpos[org_i];
+    const float3 a = frame_pos(P, P.lpos[i], org);
+    int out = 0;
+    __syncwarp();
+    for (int k0 = 0; k0 < stored; k0 += 32) {
+        const int k = k0 + lane;
+        int e = 0;
+        bool keep = k < stored;
+        if (keep) {
+            e = row[k];
+            const int j = e & (int)kRowIdxMask;
+            const float3 r = frame_pos(P, P.lpos[j], org);
+            const float r2 = fold ? frame_r2<true>(Lx, Ly, Lz, a.x, a.y, a.z, r.x, r.y, r.z)
+                                  : frame_r2<false>(Lx, Ly, Lz, a.x, a.y, a.z, r.x, r.y, r.z);
+            if (!(r2 < P.fband_lo))
+                keep = exact_r2(P.posd4[i], P.posd4[j], L, hL) < rl2;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        __syncwarp();
+        if (keep)
+            row[out + __popc(m & ((1u << lane) - 1u))] = e;
+        out += __popc(m);
+        __syncwarp();
+    }
+    return cnt - stored + out;
+}
+
+template <bool FOLD, bool SP>
+ATVB_DEV void build_share(const SysParams& P, int c, int cs, int ce, int lane,
+                          float4* __restrict__ sr, int4* __restrict__ sc, int* s_max,
+                          unsigned* s_sum) {
+    const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
+    // every field the loops use, read once: the row stores below could alias
+    // SysParams as far as the compiler knows
+    const int4* __restrict__ lp = P.lpos;
+    const int* __restrict__ cstart = P.cell_start;
+    const float sx = P.Lf_fix[0], sy = P.Lf_fix[1], sz = P.Lf_fix[2];
+    const float flo = P.fband_lo, fhi = P.fband_hi;
+    const float Lx = (float)P.L[0], Ly = (float)P.L[1], Lz = (float)P.L[2];
+    const int nc0 = P.nc[0], nc1 = P.nc[1], nc2 = P.nc[2], ncol = P.ncol;
+    const unsigned cap = (unsigned)P.cap;
+    const int4* __restrict__ cols = P.cols;
+    const int cz = c % nc2, cy = (c / nc2) % nc1, cx = c / (nc1 * nc2);
+    const int4 org = lp[cs];
+    int incl = 0, total = 0;
+    for (int i0 = cs; i0 < ce; i0 += kListAtoms) {
+        const int ni = min(kListAtoms, ce - i0);
+        __syncwarp();
+        if (lane < ni) {
+            const int4 q = lp[i0 + lane];
+            sr[lane] = make_float4((float)(int)((unsigned)q.x - (unsigned)org.x) * sx,
+                                   (float)(int)((unsigned)q.y - (unsigned)org.y) * sy,
+                                   (float)(int)((unsigned)q.z - (unsigned)org.z) * sz, 0.0f);
+        }
+        unsigned* const rows = reinterpret_cast<unsigned*>(P.nbr) + (size_t)i0 * cap;
+        unsigned off[kListAtoms]; // a * cap + the length of atom i0 + a's row so far
+#pragma unroll
+        for (int a = 0; a < kListAtoms; ++a)
+            off[a] = a * cap;
+        unsigned amb = 0; // bit a: this lane appended a candidate of the band
+        for (int c0 = 0; c0 < ncol; c0 += 32) {
+            if (ncol > 32 || i0 == cs) {
                 int a0 = 0, l0 = 0, a1 = 0, l1 = 0;
                 if (c0 + lane < ncol)
                     column_runs(nc0, nc1, nc2, cstart, cols[c0 + lane], cx, cy, cz, a0, l0,
                                 a1, l1);
                 const int tot = l0 + l1;
-                int incl = tot;
+                incl = tot;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const int t = __shfl_up_sync(full, incl, o);
                     if (lane >= o)
                         incl += t;
                 }
+                // candidate t of this column: t + x up to place y, then t + z
                 const int excl = incl - tot;
-                const int total = __shfl_sync(full, incl, 31);
-                for (int b = 0; b < total; b += 32) {
-                    const int t = b + lane;
-                    // owner column: the first lane whose inclusive sum exceeds t
-                    int own = 0;
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1) {
-                        const int probe = __shfl_sync(full, incl, own + step - 1);
-                        if (probe <= t)
-                            own += step;
-                    }
-                    own &= 31;
-                    const int o = t - __shfl_sync(full, excl, own);
-                    const int oa0 = __shfl_sync(full, a0, own);
-                    const int ol0 = __shfl_sync(full, l0, own);
-                    const int oa1 = __shfl_sync(full, a1, own);
-                    const bool live = t < total;
-                    const int j = live ? (o < ol0 ? oa0 + o : oa1 + (o - ol0)) : -1;
-                    int4 qj = make_int4(0, 0, 0, 0);
-                    if (live)
-                        qj = lp[j];
-                    if (local) {
-                        // candidate in the cell-local frame (see lframe_ok)
-                        const float rx = (float)(int)((unsigned)qj.x - (unsigned)org.x) * sx;
-                        const float ry = (float)(int)((unsigned)qj.y - (unsigned)org.y) * sy;
-                        const float rz = (float)(int)((unsigned)qj.z - (unsigned)org.z) * sz;
-                        // two atoms of the cell per pass: their screens,
-                        // votes and appends are independent, so their
-                        // latencies overlap; an odd last atom takes the
-                        // one-atom pass (sparse cells hold one atom or two)
-                        int ii = 0;
-                        for (; ii + 1 < ni; ii += 2) {
-                            const int i1 = ii + 1;
-                            const float4 ra = sr[warp][ii], rb = sr[warp][i1];
-                            const float ax = ra.x - rx, ay = ra.y - ry, az = ra.z - rz;
-                            const float bx = rb.x - rx, by = rb.y - ry, bz = rb.z - rz;
-                            const float r2a = ax * ax + ay * ay + az * az;
-                            const float r2b = bx * bx + by * by + bz * bz;
-                            const bool va = live && j != i0 + ii;
-                            const bool vb = live && j != i0 + i1;
-                            bool ha = va && r2a < flo, hb = vb && r2b < flo;
-                            const bool aa = va && !(r2a < flo) && r2a < fhi;
-                            const bool ab = vb && !(r2b < flo) && r2b < fhi;
-                            if (__any_sync(full, aa || ab)) { // rare: exact FP64 test
-                                if (aa)
-                                    ha = exact_r2(pos[i0 + ii], pos[j], L, hL) < rl2;
-                                if (ab)
-                                    hb = exact_r2(pos[i0 + i1], pos[j], L, hL) < rl2;
-                            }
-                            const unsigned ma = __ballot_sync(full, ha);
-                            const unsigned mb = __ballot_sync(full, hb);
-                            if (ma | mb) {
-                                const int basea = __shfl_sync(full, cnt, ii);
-                                const int baseb = __shfl_sync(full, cnt, i1);
-                                if (ha) {
-                                    const int wpos = basea + __popc(ma & lt);
-                                    unsigned e = (unsigned)j;
-                                    if (has_sp)
-                                        e |= special_class(P, i0 + ii, j) << 30;
-                                    if (wpos < cap)
-                                        nbr[(size_t)(i0 + ii) * cap + wpos] = (int)e;
-                                }
-                                if (hb) {
-                                    const int wpos = baseb + __popc(mb & lt);
-                                    unsigned e = (unsigned)j;
-                                    if (has_sp)
-                                        e |= special_class(P, i0 + i1, j) << 30;
-                                    if (wpos < cap)
-                                        nbr[(size_t)(i0 + i1) * cap + wpos] = (int)e;
-                                }
-                                if (lane == ii)
-                                    cnt += __popc(ma);
-                                if (lane == i1)
-                                    cnt += __popc(mb);
-                            }
-                        }
-                        if (ii < ni) {
-                            const float4 ri = sr[warp][ii];
-                            const float dx = ri.x - rx, dy = ri.y - ry, dz = ri.z - rz;
-                            const float r2f = dx * dx + dy * dy + dz * dz;
-                            const bool valid = live && j != i0 + ii;
-                            bool hit = valid && r2f < flo;
-                            const bool amb = valid && !(r2f < flo) && r2f < fhi;
-                            if (__any_sync(full, amb)) {
-                                if (amb)
-                                    hit = exact_r2(pos[i0 + ii], pos[j], L, hL) < rl2;
-                            }
-                            const unsigned m = __ballot_sync(full, hit);
-                            if (m) {
-                                const int base = __shfl_sync(full, cnt, ii);
-                                if (hit) {
-                                    const int wpos = base + __popc(m & lt);
-                                    unsigned e = (unsigned)j;
-                                    if (has_sp)
-                                        e |= special_class(P, i0 + ii, j) << 30;
-                                    if (wpos < cap)
-                                        nbr[(size_t)(i0 + ii) * cap + wpos] = (int)e;
-                                }
-                                if (lane == ii)
-                                    cnt += __popc(m);
-                            }
-                        }
-                    } else {
-                        // exact integer minimum image (small boxes)
-                        for (int ii = 0; ii < ni; ++ii) {
-                            const int4 qi = sq[warp][ii];
-                            const float dx = (float)(int)((unsigned)qi.x - (unsigned)qj.x) * sx;
-                            const float dy = (float)(int)((unsigned)qi.y - (unsigned)qj.y) * sy;
-                            const float dz = (float)(int)((unsigned)qi.z - (unsigned)qj.z) * sz;
-                            const float r2f = dx * dx + dy * dy + dz * dz;
-                            const bool valid = live && j != i0 + ii;
-                            bool hit = valid && r2f < blo;
-                            const bool amb = valid && !(r2f < blo) && r2f < bhi;
-                            if (__any_sync(full, amb)) {
-                                if (amb)
-                                    hit = exact_r2(pos[i0 + ii], pos[j], L, hL) < rl2;
-                            }
-                            const unsigned m = __ballot_sync(full, hit);
-                            if (m) {
-                                const int base = __shfl_sync(full, cnt, ii);
-                                if (hit) {
-                                    const int wpos = base + __popc(m & lt);
-                                    unsigned e = (unsigned)j;
-                                    if (has_sp)
-                                        e |= special_class(P, i0 + ii, j) << 30;
-                                    if (wpos < cap)
-                                        nbr[(size_t)(i0 + ii) * cap + wpos] = (int)e;
-                                }
-                                if (lane == ii)
-                                    cnt += __popc(m);
-                            }
-                        }
-                    }
-                }
+                __syncwarp();
+                sc[lane] = make_int4(a0 - excl, excl + l0, a1 - l0 - excl, 0);
+                total = __shfl_sync(full, incl, 31);
             }
-            if (lane < ni) {
-                const int i = i0 + lane;
-                P.nnbr[i] = cnt < cap ? cnt : cap;
-                atomicMax(&P.st->max_nnbr, cnt);
-                atomicAdd(&P.st->list_entries, (unsigned long long)cnt);
-                if (cnt > cap) {
-                    // the row is cut: pairs are missing until rows are widened
-                    atomicOr(&P.st->overflow, 1);
-                    atomicOr(&P.st->status, kStatusRowOverflow);
+            __syncwarp();
+            // candidate t = b + lane of the window, and its position
+            auto fetch = [&](int b, int4& q) {
+                const int t = b + lane;
+                // owner column: the first lane whose inclusive sum exceeds t
+                int own = 0;
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) {
+                    const int probe = __shfl_sync(full, incl, own + step - 1);
+                    if (probe <= t)
+                        own += step;
+                }
+                const int4 k = sc[own & 31];
+                const int j = t < total ? (t < k.y ? t + k.x : t + k.z) : -1;
+                if (j >= 0)
+                    q = lp[j];
+                return j;
+            };
+            int4 qn = make_int4(0, 0, 0, 0);
+            int jn = total > 0 ? fetch(0, qn) : -1;
+            for (int b = 0; b < total; b += 32) {
+                const int j = jn;
+                const int4 q = qn;
+                if (b + 32 < total)
+                    jn = fetch(b + 32, qn);
+                float rx = (float)(int)((unsigned)q.x - (unsigned)org.x) * sx;
+                const float ry = (float)(int)((unsigned)q.y - (unsigned)org.y) * sy;
+                const float rz = (float)(int)((unsigned)q.z - (unsigned)org.z) * sz;
+                if (j < 0)
+                    rx = __int_as_float(0x7fc00000); // NaN: never a hit
+                const int jrel = j - i0; // == a: the atom itself
+#pragma unroll
+                for (int a = 0; a < kListAtoms; ++a) {
+                    if (a >= ni)
+                        break; // warp-uniform
+                    const float4 r = sr[a];
+                    const float r2 = frame_r2<FOLD>(Lx, Ly, Lz, r.x, r.y, r.z, rx, ry, rz);
+                    // no branches but the one on a: a divergent region costs
+                    // more than the few instructions it would skip
+                    const bool hit = r2 < fhi && jrel != a;
+                    const unsigned m = __ballot_sync(full, hit);
+                    const unsigned w = off[a] + (unsigned)__popc(m & lt);
+                    amb = hit && !(r2 < flo) ? amb | (1u << a) : amb;
+                    unsigned e = (unsigned)j;
+                    if (SP && hit)
+                        e |= special_class(P, i0 + a, j) << 30;
+                    if (hit && w < (a + 1u) * cap)
+                        rows[w] = e;
+                    off[a] += (unsigned)__popc(m);
                 }
             }
         }
+        amb = __reduce_or_sync(full, amb);
+        int cnt = 0; // row length of atom i0 + lane
+#pragma unroll
+        for (int a = 0; a < kListAtoms; ++a) {
+            if (a >= ni)
+                break;
+            int len = (int)(off[a] - a * cap);
+            if (amb & (1u << a))
+                len = settle_row(P, i0 + a, cs, len);
+            if (lane == a)
+                cnt = len;
+        }
+        const int wmax = __reduce_max_sync(full, cnt);
+        const int wsum = __reduce_add_sync(full, cnt);
+        if (lane == 0) {
+            atomicMax(s_max, wmax);
+            atomicAdd(s_sum, (unsigned)wsum);
+        }
+        if (lane < ni) {
+            P.nnbr[i0 + lane] = min(cnt, (int)cap);
+            if (cnt > (int)cap) {
+                // the row is cut: pairs are missing until rows are widened
+                atomicOr(&P.st->overflow, 1);
+                atomicOr(&P.st->status, kStatusRowOverflow);
+            }
+        }
     }
+}
+
+__global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
+    k_build_list(const Item* items, int nitems, const SysParams* sp, int split_log2) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ float4 sr[kListWarps][kListAtoms];
+    __shared__ int4 sc[kListWarps][32];
+    // the longest row and the number of entries of the rows built so far by
+    // this block, added to the system once per block and system (one atomic
+    // of each per atom serialises on one address: 2,000,376 of them took
+    // 0.5 ms of the build of 1,000,188 LJ atoms)
+    __shared__ int s_max;
+    __shared__ unsigned s_sum;
+    int cur = -1;
+    auto flush = [&] { // block-uniform
+        __syncthreads();
+        if (threadIdx.x == 0 && cur >= 0) {
+            SysState* st = sp[cur].st;
+            if (s_max > 0)
+                atomicMax(&st->max_nnbr, s_max);
+            if (s_sum)
+                atomicAdd(&st->list_entries, (unsigned long long)s_sum);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_max = 0;
+            s_sum = 0;
+        }
+        __syncthreads();
+    };
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const Item item = items[it];
+        const SysParams& P = sp[item.sys];
+        if (!P.st->rebuild)
+            continue;
+        if (item.sys != cur) {
+            flush();
+            cur = item.sys;
+        }
+        const int task = item.begin + warp;
+        const int c = task >> split_log2;
+        if (c >= P.ncell)
+            continue; // warp-uniform
+        // this warp's share of the cell's atoms
+        const int c_lo = P.cell_start[c], c_n = P.cell_start[c + 1] - c_lo;
+        const int part = task & ((1 << split_log2) - 1);
+        const int cs = c_lo + ((c_n * part) >> split_log2);
+        const int ce = c_lo + ((c_n * (part + 1)) >> split_log2);
+        if (cs >= ce)
+            continue;
+        if (P.lframe_ok) {
+            if (P.has_special)
+                build_share<false, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum);
+            else
+                build_share<false, false>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max,
+                                          &s_sum);
+        } else {
+            if (P.has_special)
+                build_share<true, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum);
+            else
+                build_share<true, false>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max,
+                                         &s_sum);
+        }
+    }
+    if (cur >= 0)
+        flush();
 }
 
 // Binning and the sorted repack: after these the sorted positions (pos4)
@@ -472,17 +565,16 @@ __global__ void __launch_bounds__(256)
 void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s) {
     k_cell_count<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
                                                    lc.sp);
-    k_cell_scan<<<lc.nsys, 1024, 0, s>>>(lc.sys_list, lc.sp);
+    k_cell_sums<<<lc.scan.grid, kChunk, 0, s>>>(lc.scan.d, lc.scan.n, lc.sp);
+    k_cell_scan<<<lc.scan.grid, kChunk, 0, s>>>(lc.scan.d, lc.scan.n, lc.sp);
     k_cell_scatter<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
                                                      lc.sp);
-    k_cell_sort<<<lc.cells.grid, kChunk, 0, s>>>(lc.cells.d, lc.cells.n,
-                                                  lc.sp);
     k_permute<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n, lc.sp);
 }
 
 void launch_build_list(const LaunchCfg& lc, cudaStream_t s) {
-    k_build_list<<<lc.list.grid, 32 * kListChunk, 0, s>>>(lc.list.d,
-                                                           lc.list.n, lc.sp);
+    k_build_list<<<lc.list.grid, 32 * kListChunk, 0, s>>>(lc.list.d, lc.list.n, lc.sp,
+                                                           lc.list_split_log2);
 }
 
 void launch_rebuild(const LaunchCfg& lc, cudaStream_t s) {
