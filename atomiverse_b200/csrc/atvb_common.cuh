@@ -248,6 +248,10 @@ struct SysParams {
     int *perm, *rank, *cell_of, *slot, *cell_count, *cell_start;
     int* cell_sums; // atoms per kScanChunk cells
     int2* perm0;    // {atom, fixed-point z} by cell, in arrival order (k_cell_scatter)
+    int small_sort; // the whole cell sort in one block (k_sort_small)
+    // finished items of k_integrate_a / k_integrate_b: the block that
+    // completes the last one runs the system's scalar updates
+    unsigned* tickets;
     int *nbr, *nnbr;
     // PME buffers
     unsigned long long* grid_fix;
@@ -284,6 +288,16 @@ ATVB_DEV void red_add_u64(unsigned long long* a, unsigned long long v) {
 
 ATVB_DEV void fix_add(unsigned long long* a, double v) {
     red_add_u64(a, (unsigned long long)to_fix(v));
+}
+
+// Programmatic dependent launch: every kernel of the step first lets the next
+// one start launching, then waits until the ones before it have finished and
+// their writes are visible (no-ops for a kernel launched without the
+// attribute).  No thread may read or write, or leave, before the wait: the
+// next kernel's own wait covers this grid only.
+ATVB_DEV void pdl_sync() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename T>

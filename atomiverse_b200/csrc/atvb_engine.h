@@ -161,6 +161,7 @@ class Engine {
     void clear_profile() { prof_acc_.clear(); }
     int64_t last_launches() const { return last_launches_; }
     int64_t kernels_per_step() const;
+    int64_t rebuild_kernels() const;
     cudaStream_t stream() const { return stream_; }
     int device() const { return device_; }
     int lanes() const { return lc_.pair_G; }
@@ -179,7 +180,9 @@ class Engine {
     bool check_lists(const LaunchCfg& lc);
     void sized_rebuild(const LaunchCfg& lc);
     LaunchCfg restricted_cfg(int id);
-    void enqueue_step(bool profile);
+    void enqueue_step(bool profile, bool first, bool last);
+    bool merge_halves() const;
+    cudaGraphExec_t capture_steps(int steps);
     void widen_rows();
     int deform_budget(int n);
     void run_steps(int n);
@@ -225,10 +228,12 @@ class Engine {
     bool dirty_ = true;
     int list_epoch_ = 0;
     std::map<int, std::pair<int, LaunchCfg>> single_;
-    cudaGraph_t graph_ = nullptr;
-    cudaGraphExec_t gexec_ = nullptr;
+    cudaGraphExec_t gexec_ = nullptr;      // one step
+    cudaGraphExec_t gexec_many_ = nullptr; // kManySteps steps
+    long long graph_steps_ = 0;            // steps run since the graphs were captured
     int lanes_fixed_ = 0;
     int64_t last_launches_ = 0;
+    int64_t merged_ = 0; // launches of the current call saved by k_integrate_ba
     int64_t steps_since_check_ = 0;
     bool profiling_ = false;
     std::vector<cudaEvent_t> prof_events_;

@@ -9,11 +9,12 @@
 namespace atvb {
 
 constexpr int kChunk = 256;     // atoms per item of the per-atom kernels
-constexpr int kRebuildKernels = 6; // launches of one list build (cell sort + rows)
 constexpr long long kCondMinAtoms = 100000; // engines from this size skip them by
                                             // conditional graph nodes
 constexpr int kListChunk = 4;   // warp tasks per item of the list build
 constexpr int kScanChunk = 2048; // cells per item of the cell scan
+// largest system whose cell sort runs in one block (k_sort_small)
+constexpr int kSortSmallAtoms = 8192, kSortSmallCells = 16384;
 constexpr int kGridChunk = 4096; // grid points per item of the PME grid kernels
 constexpr int kLaneClasses = 6;  // pair lanes per atom: 1, 2, 4, 8, 16, 32
 constexpr int kGenLanes = 8;      // lanes per atom of k_pair_general
@@ -56,7 +57,15 @@ struct LaunchCfg {
     ItemList pair[2][kLaneClasses];
     ItemList pair_gen[2]; // [precision]: systems with types or special pairs
                           // (kChunk / kGenLanes atoms per item)
-    ItemList scan;      // kScanChunk cells per item
+    // the cell sort: systems sorted by one block each (small_list, nsmall;
+    // small_smem bytes for the largest), and the items of the others
+    const int* small_list = nullptr;
+    int nsmall = 0;
+    size_t small_smem = 0;
+    ItemList sort_atoms; // kChunk atoms per item
+    ItemList scan;       // kScanChunk cells per item
+    // kernels of the chain launched as programmatic dependents (step graphs)
+    bool pdl = false;
     ItemList pme_atoms; // kChunk atoms of PME systems
     ItemList pme_grid;  // kGridChunk half-complex grid points per item
     ItemList pme_real;  // kGridChunk real grid points per item
@@ -72,17 +81,41 @@ struct LaunchCfg {
     int pme_mixed = 0;
 };
 
-// neighbor.cu
-void launch_rebuild(const LaunchCfg& lc, cudaStream_t s);
-void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s);
-void launch_build_list(const LaunchCfg& lc, cudaStream_t s);
-// pair.cu
-void launch_pair(const LaunchCfg& lc, cudaStream_t s);
-void launch_pair_fix(const LaunchCfg& lc, cudaStream_t s);
-// pair_general.cu
-void launch_pair_general(const LaunchCfg& lc, cudaStream_t s);
 void cuda_check(cudaError_t e, const char* what); // engine.cu: throws on error
 
+// A launch on stream s; `pdl`: as a programmatic dependent of the kernel
+// before it in the stream (which must be a kernel that calls pdl_sync), so
+// that its blocks are set up while that one drains.
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
+                     bool pdl, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cuda_check(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...), "kernel launch");
+}
+
+// neighbor.cu
+bool small_sort_fits(int n, int ncell);
+size_t small_sort_smem(int n, int ncell);
+void sort_smem_optin();
+void launch_rebuild(const LaunchCfg& lc, cudaStream_t s);
+// `pdl` of a launcher: whether its first kernel depends on the launch before
+// it alone (the rest of its chain follows lc.pdl)
+void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s, bool pdl = false);
+void launch_build_list(const LaunchCfg& lc, cudaStream_t s, bool pdl = false);
+// pair.cu
+void launch_pair(const LaunchCfg& lc, cudaStream_t s, bool pdl = false);
+void launch_pair_fix(const LaunchCfg& lc, cudaStream_t s);
+// pair_general.cu
+void launch_pair_general(const LaunchCfg& lc, cudaStream_t s, bool pdl = false);
 // pme.cu
 void launch_pme_spread(const LaunchCfg& lc, cudaStream_t s);
 void launch_pme_gather(const LaunchCfg& lc, cudaStream_t s);
@@ -98,16 +131,20 @@ int fft_reg_index(int n);
 int fft_reg_lines(int idx, bool mixed);
 int fft_reg_cols(bool mixed);
 void launch_fft_reg(int pass, int idx, bool mixed, const ItemList& il, const SysParams* sp,
-                    cudaStream_t s);
+                    cudaStream_t s, bool pdl);
 // integrate.cu
-void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s);
-// cond_sort / cond_rows / use_cond: the step graph's conditional handles of
-// the list build (set when a system rebuilds), only while the step is being
-// captured
-void launch_sys_a(const LaunchCfg& lc, cudaStream_t s, cudaGraphConditionalHandle cond_sort = 0,
-                  cudaGraphConditionalHandle cond_rows = 0, bool use_cond = false);
-void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s);
+// fuse: the scalar updates of k_sys_a / k_sys_b run in the last block of each
+// system instead of a launch of their own.  cond_sort / cond_rows / use_cond:
+// the step graph's conditional handles of the list build (set when a system
+// rebuilds), only while the step is being captured
+void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse = false, bool pdl = false,
+                        cudaGraphConditionalHandle cond_sort = 0,
+                        cudaGraphConditionalHandle cond_rows = 0, bool use_cond = false);
+void launch_sys_a(const LaunchCfg& lc, cudaStream_t s);
+void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s, bool fuse = false, bool pdl = false);
+void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool pdl);
 void launch_sys_b(const LaunchCfg& lc, cudaStream_t s);
+void launch_baro(const LaunchCfg& lc, cudaStream_t s);
 void launch_sys_energy(const LaunchCfg& lc, cudaStream_t s);
 void launch_force_rebuild(const LaunchCfg& lc, cudaStream_t s);
 void launch_state_in(const LaunchCfg& lc, cudaStream_t s);

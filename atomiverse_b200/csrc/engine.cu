@@ -332,6 +332,7 @@ void Slot::replan_cells(double shrink) {
         hp.npt_Lmin[k] = geo.Lmin[k];
     }
     hp.ncell = geo.nc[0] * geo.nc[1] * geo.nc[2];
+    hp.small_sort = small_sort_fits(hp.n, hp.ncell) ? 1 : 0;
     hp.ncol = (int)geo.cols.size();
     hp.cell_count = (int*)dalloc(sizeof(int) * hp.ncell);
     hp.cell_start = (int*)dalloc(sizeof(int) * (hp.ncell + 1));
@@ -523,6 +524,9 @@ Slot::Slot(const atvb_system_desc& d, const DevMem& mem) : desc(d), mem_(mem) {
     hp.cell_of = di(n);
     hp.slot = di(n);
     hp.perm0 = (int2*)dalloc((size_t)n * sizeof(int2));
+    hp.small_sort = small_sort_fits(n, hp.ncell) ? 1 : 0;
+    hp.tickets = (unsigned*)dalloc(2 * sizeof(unsigned));
+    CK(cudaMemsetAsync(hp.tickets, 0, 2 * sizeof(unsigned), stream));
     hp.nnbr = di(n);
     hp.cell_count = di(hp.ncell);
     hp.cell_start = di(hp.ncell + 1);
@@ -641,6 +645,7 @@ Engine::Engine(int device) : device_(device) {
     CK(cudaEventCreateWithFlags(&pme_join_, cudaEventDisableTiming));
     // the FFT blocks' line buffers live in dynamic shared memory above 48 KB
     fft_smem_optin(kFftSmem + 1024);
+    sort_smem_optin();
 }
 
 Engine::~Engine() {
@@ -676,12 +681,12 @@ Engine::~Engine() {
 }
 
 void Engine::release_graph() {
-    if (gexec_)
-        cudaGraphExecDestroy(gexec_);
-    if (graph_)
-        cudaGraphDestroy(graph_);
-    gexec_ = nullptr;
-    graph_ = nullptr;
+    for (cudaGraphExec_t* g : {&gexec_, &gexec_many_}) {
+        if (*g)
+            cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+    graph_steps_ = 0;
 }
 
 int Engine::add(const atvb_system_desc& d) {
@@ -868,8 +873,9 @@ void Engine::build_lists() {
     for (void* p : list_allocs_)
         mem_.free(p);
     list_allocs_.clear();
-    std::vector<Item> atoms, list, scan, patoms;
-    std::vector<int> sys;
+    std::vector<Item> atoms, list, sort_atoms, scan, patoms;
+    std::vector<int> sys, small;
+    size_t small_smem = 0;
     std::vector<Item> pair_by[2][kLaneClasses];
     std::vector<Item> pair_gen[2];
     lc_ = LaunchCfg{};
@@ -908,8 +914,15 @@ void Engine::build_lists() {
             for (int b = 0; b < P.n; b += kPairBlock / sp->lanes)
                 pv.push_back({k, b});
         }
-        for (int b = 0; b < P.ncell; b += kScanChunk)
-            scan.push_back({k, b});
+        if (P.small_sort) {
+            small.push_back(k);
+            small_smem = std::max(small_smem, small_sort_smem(P.n, P.ncell));
+        } else {
+            for (int b = 0; b < P.n; b += kChunk)
+                sort_atoms.push_back({k, b});
+            for (int b = 0; b < P.ncell; b += kScanChunk)
+                scan.push_back({k, b});
+        }
         if (P.prec == kMixed)
             lc_.any_mixed = 1;
         else
@@ -941,7 +954,17 @@ void Engine::build_lists() {
             lc_.pair[p][c] = make_list(list_allocs_, pair_by[p][c], num_sms_ * 16, mem_);
     for (int p = 0; p < 2; ++p)
         lc_.pair_gen[p] = make_list(list_allocs_, pair_gen[p], num_sms_ * 16, mem_);
+    lc_.sort_atoms = make_list(list_allocs_, sort_atoms, g_light, mem_);
     lc_.scan = make_list(list_allocs_, scan, g_light, mem_);
+    lc_.nsmall = (int)small.size();
+    lc_.small_smem = small_smem;
+    if (!small.empty()) {
+        void* p = mem_.alloc(sizeof(int) * small.size());
+        list_allocs_.push_back(p);
+        CK(cudaMemcpyAsync(p, small.data(), sizeof(int) * small.size(), cudaMemcpyHostToDevice,
+                           stream_));
+        lc_.small_list = (const int*)p;
+    }
     lc_.pme_atoms = make_list(list_allocs_, patoms, g_light, mem_);
     lc_.nsys = (int)sys.size();
     if (!sys.empty()) {
@@ -1139,6 +1162,7 @@ void Engine::enqueue_step_components() {
     phase(ATVB_PHASE_FINAL_INTEGRATE, [&] { launch_integrate_b(lc_, stream_); });
     phase(ATVB_PHASE_END_OF_STEP, [&] {
         launch_sys_b(lc_, stream_);
+        launch_baro(lc_, stream_);
         if (lc_.any_snap)
             launch_snapshots(lc_, stream_);
     });
@@ -1147,10 +1171,15 @@ void Engine::enqueue_step_components() {
 }
 
 // Kernel launches of one step.
+// Launches of one list build: the cell sorts and the rows.
+int64_t Engine::rebuild_kernels() const {
+    return (lc_.nsmall ? 1 : 0) + (lc_.sort_atoms.n ? 5 : 0) + 1;
+}
+
 int64_t Engine::kernels_per_step() const {
     int64_t k = 0;
-    k += 2;                                   // integrate_a, sys_a
-    k += kRebuildKernels;                     // list build (rebuild steps only)
+    k += 1;                                   // integrate_a (with the scalar updates)
+    k += rebuild_kernels();                   // list build (rebuild steps only)
     for (int p = 0; p < 2; ++p)                // pair: one per lane class used
         for (int c = 0; c < kLaneClasses; ++c)
             k += lc_.pair[p][c].n ? 1 : 0;
@@ -1158,7 +1187,8 @@ int64_t Engine::kernels_per_step() const {
     k += (lc_.pair_gen[0].n ? 1 : 0) + (lc_.pair_gen[1].n ? 1 : 0); // general pair
     if (!pme_slots_.empty())
         k += 2 + lc_.fft.launches();          // spread, gather, the transform passes
-    k += 2;                                   // integrate_b, sys_b
+    k += 1;                                   // integrate_b (with the scalar updates)
+    k += comps_.empty() ? 0 : 2;              // the scalar updates as their own kernels
     k += lc_.any_snap ? 3 : 0;                // trajectory snapshots
     k += lc_.any_baro ? 1 : 0;                // Berendsen position scaling
     return k;
@@ -1172,6 +1202,9 @@ int64_t Engine::kernels_per_step() const {
 void Engine::enqueue_forces(const LaunchCfg& lc, const std::vector<int>& pme,
                             bool profile, bool overlap, bool build_list) {
     const bool side = overlap && !profile && !pme.empty();
+    // programmatic launches: within the step graph, after a kernel of the
+    // same stream that is the launch's only predecessor
+    bool chain = lc.pdl && !capturing_;
     cudaStream_t ps = side ? pme_stream_ : stream_;
     if (side) {
         CK(cudaEventRecord(pme_fork_, stream_));
@@ -1185,7 +1218,7 @@ void Engine::enqueue_forces(const LaunchCfg& lc, const std::vector<int>& pme,
         if (capturing_)
             capture_if(cond_rows_, [&](cudaStream_t cs) { launch_build_list(lc, cs); });
         else
-            launch_build_list(lc, stream_);
+            launch_build_list(lc, stream_, chain);
     }
     if (!pme.empty()) {
         prof_mark(profile, "pme_spread");
@@ -1196,7 +1229,7 @@ void Engine::enqueue_forces(const LaunchCfg& lc, const std::vector<int>& pme,
         launch_pme_gather(lc, ps);
     }
     prof_mark(profile, "pair");
-    launch_pair(lc, stream_);
+    launch_pair(lc, stream_, chain);
     if (lc.any_near) {
         prof_mark(profile, "pair_fix");
         launch_pair_fix(lc, stream_);
@@ -1241,14 +1274,9 @@ void Engine::capture_if(cudaGraphConditionalHandle h, F&& body) {
 // ions +0.8 %, 1,000,188 LJ atoms +7 %; but 4,000 and 10,648 atoms -13 %
 // and -15 % (the conditional nodes cost more than the early-exit launches
 // of a small system), hence the threshold.
-void Engine::enqueue_step(bool profile) {
-    if (capturing_) {
-        long long atoms = 0;
-        for (const auto& up : slots_)
-            if (up)
-                atoms += up->hp.n;
-        capturing_ = atoms >= kCondMinAtoms;
-    }
+void Engine::enqueue_step(bool profile, bool first, bool last) {
+    const bool pdl = lc_.pdl, merge = !profile && merge_halves();
+    const bool after_b = pdl && !first && !lc_.any_baro && !lc_.any_snap;
     if (capturing_) {
         cudaStreamCaptureStatus st;
         unsigned long long id = 0;
@@ -1258,17 +1286,25 @@ void Engine::enqueue_step(bool profile) {
         CK(cudaGraphConditionalHandleCreate(&cond_rows_, g, 0, cudaGraphCondAssignDefault));
     }
     prof_mark(profile, "integrate_a");
-    launch_integrate_a(lc_, stream_);
-    launch_sys_a(lc_, stream_, cond_sort_, cond_rows_, capturing_);
+    if (first || !merge)
+        launch_integrate_a(lc_, stream_, true, after_b, cond_sort_, cond_rows_, capturing_);
     prof_mark(profile, "neighbor");
     if (capturing_)
-        capture_if(cond_sort_, [&](cudaStream_t cs) { launch_sort_cells(lc_, cs); });
+        capture_if(cond_sort_, [&](cudaStream_t cs) {
+            LaunchCfg plain = lc_; // no programmatic edges in a conditional body
+            plain.pdl = false;
+            launch_sort_cells(plain, cs);
+        });
     else
-        launch_sort_cells(lc_, stream_);
+        launch_sort_cells(lc_, stream_, pdl);
     enqueue_forces(lc_, pme_slots_, profile, true, true);
     prof_mark(profile, "integrate_b");
-    launch_integrate_b(lc_, stream_);
-    launch_sys_b(lc_, stream_);
+    const bool after_pair = pdl && pme_slots_.empty();
+    if (last || !merge)
+        launch_integrate_b(lc_, stream_, true, after_pair);
+    else
+        launch_integrate_ba(lc_, stream_, after_pair);
+    launch_baro(lc_, stream_);
     if (lc_.any_snap) {
         prof_mark(profile, "snapshot");
         launch_snapshots(lc_, stream_);
@@ -1368,6 +1404,7 @@ void Engine::run_pieces(int n, double* step_ms, double* total_ms) {
     std::vector<cudaEvent_t> ev;
     double tot = 0.0;
     int left = n, done = 0;
+    merged_ = 0;
     do {
         // The cell re-plan and the row check read what the previous call
         // left (the engine stream is non-blocking, so a plain copy would not
@@ -1421,19 +1458,43 @@ void Engine::run_pieces(int n, double* step_ms, double* total_ms) {
         cudaEventDestroy(e);
     if (timed)
         *total_ms = tot;
-    last_launches_ = kernels_per_step() * done;
+    last_launches_ = kernels_per_step() * done - merged_;
     steps_since_check_ += done;
 }
 
-void Engine::ensure_graph() {
-    if (gexec_)
-        return;
+// Whether a graph of several steps may run the final half of a step and the
+// initial half of the next in one kernel (k_integrate_ba).
+bool Engine::merge_halves() const {
+    for (const auto& up : slots_) {
+        if (!up || !up->uploaded)
+            continue;
+        const SysParams& P = up->hp;
+        if ((P.thermostat != kNVE && P.thermostat != kLangevin) || P.generic_drift || P.baro ||
+            P.deform_axis >= 0 || P.stop_on_nan || P.snap_ring || P.ext_f)
+            return false;
+    }
+    return !capturing_; // conditional build nodes: k_integrate_a sets them
+}
+
+// The step graph: `steps` steps, captured from stream_.
+cudaGraphExec_t Engine::capture_steps(int steps) {
+    long long atoms = 0;
+    for (const auto& up : slots_)
+        if (up)
+            atoms += up->hp.n;
+    cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    capturing_ = true;
+    capturing_ = atoms >= kCondMinAtoms;
+    // programmatic launches only where a kernel does not fill the GPU: the
+    // waiting blocks of the PME chain's next kernel would hold slots that
+    // the pair kernel beside it can use (262,144 ions 2 % slower with them)
+    lc_.pdl = !capturing_;
     try {
-        enqueue_step(false);
+        for (int k = 0; k < steps; ++k)
+            enqueue_step(false, k == 0, k == steps - 1);
     } catch (...) {
         capturing_ = false;
+        lc_.pdl = false;
         cudaGraph_t g = nullptr;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(cond_stream_, &cs) == cudaSuccess &&
@@ -1449,9 +1510,25 @@ void Engine::ensure_graph() {
         throw;
     }
     capturing_ = false;
-    CK(cudaStreamEndCapture(stream_, &graph_));
-    CK(cudaGraphInstantiate(&gexec_, graph_, 0));
+    lc_.pdl = false;
+    CK(cudaStreamEndCapture(stream_, &graph));
+    cudaGraphExec_t exec = nullptr;
+    const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph); // the executable graph keeps its own copy
+    CK(e);
+    return exec;
 }
+
+void Engine::ensure_graph() {
+    if (!gexec_)
+        gexec_ = capture_steps(1);
+}
+
+// Steps per launch of the longer graph a small engine gets once its work
+// lists have stood for kManyAfter steps (a server whose requests come and go
+// recaptures too often to pay for it): its programmatic launches also reach
+// from one step into the next.
+constexpr int kManySteps = 8, kManyAfter = 24;
 
 void Engine::run_steps(int n) {
     if (!comps_.empty()) {
@@ -1462,14 +1539,28 @@ void Engine::run_steps(int n) {
     }
     if (profiling_) {
         for (int k = 0; k < n; ++k) {
-            enqueue_step(true);
+            enqueue_step(true, true, true);
             CK(cudaGetLastError());
         }
         collect_profile();
     } else {
         ensure_graph();
-        for (int k = 0; k < n; ++k)
+        long long atoms = 0;
+        for (const auto& up : slots_)
+            if (up)
+                atoms += up->hp.n;
+        int k = 0;
+        if (atoms < kCondMinAtoms && n >= kManySteps && graph_steps_ >= kManyAfter) {
+            if (!gexec_many_)
+                gexec_many_ = capture_steps(kManySteps);
+            for (; k + kManySteps <= n; k += kManySteps) {
+                CK(cudaGraphLaunch(gexec_many_, stream_));
+                merged_ += merge_halves() ? kManySteps - 1 : 0;
+            }
+        }
+        for (; k < n; ++k)
             CK(cudaGraphLaunch(gexec_, stream_));
+        graph_steps_ += n;
     }
 }
 
@@ -1624,14 +1715,17 @@ LaunchCfg Engine::restricted_cfg(int id) {
         return it->second.second;
     Slot* s = slot(id);
     const SysParams& P = s->hp;
-    std::vector<Item> atoms, list, scan, pair, patoms;
+    std::vector<Item> atoms, list, sort_atoms, scan, pair, patoms;
     for (int b = 0; b < P.n; b += kChunk)
         atoms.push_back({id, b});
     const int split = list_split(P.ncell, P.n, num_sms_);
     for (long long b = 0; b < (long long)P.ncell << split; b += kListChunk)
         list.push_back({id, (int)b});
-    for (int b = 0; b < P.ncell; b += kScanChunk)
-        scan.push_back({id, b});
+    if (!P.small_sort) {
+        sort_atoms = atoms;
+        for (int b = 0; b < P.ncell; b += kScanChunk)
+            scan.push_back({id, b});
+    }
     const int pchunk = kPairBlock / (P.general ? kGenLanes : s->lanes);
     for (int b = 0; b < P.n; b += pchunk)
         pair.push_back({id, b});
@@ -1643,6 +1737,7 @@ LaunchCfg Engine::restricted_cfg(int id) {
     c.atoms = make_list(list_allocs_, atoms, num_sms_ * 16, mem_);
     c.list = make_list(list_allocs_, list, num_sms_ * 32, mem_);
     c.list_split_log2 = split;
+    c.sort_atoms = make_list(list_allocs_, sort_atoms, num_sms_ * 16, mem_);
     c.scan = make_list(list_allocs_, scan, num_sms_ * 16, mem_);
     for (int p = 0; p < 2; ++p) {
         for (int k = 0; k < kLaneClasses; ++k)
@@ -1670,6 +1765,9 @@ LaunchCfg Engine::restricted_cfg(int id) {
     CK(cudaStreamSynchronize(stream_));
     c.sys_list = (const int*)p;
     c.nsys = 1;
+    c.nsmall = P.small_sort ? 1 : 0;
+    c.small_list = c.sys_list;
+    c.small_smem = small_sort_smem(P.n, P.ncell);
     single_[id] = {list_epoch_, c};
     return c;
 }
@@ -1854,6 +1952,7 @@ void Engine::set_stop_on_nan(int id, bool on) {
     s->hp.stop_on_nan = on ? 1 : 0;
     push_params(id);
     CK(cudaStreamSynchronize(stream_));
+    release_graph(); // a system that may stop keeps its half steps apart
 }
 
 // Capacity overrides: a pinned row length (0: automatic) and the size of

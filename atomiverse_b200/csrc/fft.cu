@@ -248,6 +248,7 @@ ATVB_DEV void load_fac(const SysParams& P, int axis, int* s_fac, int& nf) {
 template <bool MIXED>
 __global__ void __launch_bounds__(kFftBlock, 3)
     k_fft_zf(const Item* items, int nitems, const SysParams* sp, int C) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename Cplx<T>::type;
     extern __shared__ unsigned char fsh_raw[];
@@ -317,6 +318,7 @@ __global__ void __launch_bounds__(kFftBlock, 3)
 template <bool MIXED, bool INV>
 __global__ void __launch_bounds__(kFftBlock, 3)
     k_fft_y(const Item* items, int nitems, const SysParams* sp, int C) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename Cplx<T>::type;
     extern __shared__ unsigned char fsh_raw[];
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(kFftBlock, 3)
 template <bool MIXED>
 __global__ void __launch_bounds__(kFftBlock, 3)
     k_fft_x_infl(const Item* items, int nitems, const SysParams* sp, int C) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename Cplx<T>::type;
     extern __shared__ unsigned char fsh_raw[];
@@ -446,6 +449,7 @@ __global__ void __launch_bounds__(kFftBlock, 3)
 template <bool MIXED>
 __global__ void __launch_bounds__(kFftBlock, 3)
     k_fft_zi(const Item* items, int nitems, const SysParams* sp, int C) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename Cplx<T>::type;
     extern __shared__ unsigned char fsh_raw[];
@@ -516,22 +520,25 @@ static size_t fft_smem(int C, int n, int K, bool mixed) {
 // there is one, else the generic Stockham kernel above.
 template <bool MIXED>
 static void fft_pass(int pass, const std::vector<FftGroup>& gs, const SysParams* sp,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool pdl) {
     for (const FftGroup& g : gs) {
         if (g.items.n == 0)
             continue;
         if (g.reg >= 0) {
-            launch_fft_reg(pass, g.reg, MIXED, g.items, sp, s);
+            launch_fft_reg(pass, g.reg, MIXED, g.items, sp, s, pdl);
             continue;
         }
         const size_t sm = fft_smem(g.c, g.n, g.k, MIXED);
         const ItemList& il = g.items;
+        auto go = [&](auto kernel) {
+            launch_k(kernel, il.grid, kFftBlock, sm, s, pdl, il.d, il.n, sp, g.c);
+        };
         switch (pass) {
-        case 0: k_fft_zf<MIXED><<<il.grid, kFftBlock, sm, s>>>(il.d, il.n, sp, g.c); break;
-        case 1: k_fft_y<MIXED, false><<<il.grid, kFftBlock, sm, s>>>(il.d, il.n, sp, g.c); break;
-        case 2: k_fft_x_infl<MIXED><<<il.grid, kFftBlock, sm, s>>>(il.d, il.n, sp, g.c); break;
-        case 3: k_fft_y<MIXED, true><<<il.grid, kFftBlock, sm, s>>>(il.d, il.n, sp, g.c); break;
-        default: k_fft_zi<MIXED><<<il.grid, kFftBlock, sm, s>>>(il.d, il.n, sp, g.c); break;
+        case 0: go(k_fft_zf<MIXED>); break;
+        case 1: go(k_fft_y<MIXED, false>); break;
+        case 2: go(k_fft_x_infl<MIXED>); break;
+        case 3: go(k_fft_y<MIXED, true>); break;
+        default: go(k_fft_zi<MIXED>); break;
         }
     }
 }
@@ -539,11 +546,11 @@ static void fft_pass(int pass, const std::vector<FftGroup>& gs, const SysParams*
 template <bool MIXED>
 static void fft_all(const LaunchCfg& lc, cudaStream_t s) {
     const FftCfg& f = lc.fft;
-    fft_pass<MIXED>(0, f.z, lc.sp, s);
-    fft_pass<MIXED>(1, f.y, lc.sp, s);
-    fft_pass<MIXED>(2, f.x, lc.sp, s);
-    fft_pass<MIXED>(3, f.y, lc.sp, s);
-    fft_pass<MIXED>(4, f.z, lc.sp, s);
+    fft_pass<MIXED>(0, f.z, lc.sp, s, lc.pdl);
+    fft_pass<MIXED>(1, f.y, lc.sp, s, lc.pdl);
+    fft_pass<MIXED>(2, f.x, lc.sp, s, lc.pdl);
+    fft_pass<MIXED>(3, f.y, lc.sp, s, lc.pdl);
+    fft_pass<MIXED>(4, f.z, lc.sp, s, lc.pdl);
 }
 
 void launch_pme_fft(const LaunchCfg& lc, cudaStream_t s) {

@@ -273,6 +273,7 @@ template <int N1, int N2, bool MIXED>
 __global__ void __launch_bounds__(Shape<N1, N2>::template z_threads<MIXED>(),
                                   min_blocks(Shape<N1, N2>::template z_threads<MIXED>(), 80))
     k_fftr_zf(const Item* items, int nitems, const SysParams* sp) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename C2<T>::type;
     using S = Shape<N1, N2>;
@@ -345,6 +346,7 @@ __global__ void __launch_bounds__(Shape<N1, N2>::template col_threads<MIXED>(),
                                   min_blocks(Shape<N1, N2>::template col_threads<MIXED>(),
                                              MIXED ? 64 : 96))
     k_fftr_y(const Item* items, int nitems, const SysParams* sp) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename C2<T>::type;
     using S = Shape<N1, N2>;
@@ -396,6 +398,7 @@ template <int N1, int N2, bool MIXED>
 __global__ void __launch_bounds__(Shape<N1, N2>::template col_threads<MIXED>(),
                                   min_blocks(Shape<N1, N2>::template col_threads<MIXED>(), 128))
     k_fftr_x(const Item* items, int nitems, const SysParams* sp) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename C2<T>::type;
     using S = Shape<N1, N2>;
@@ -520,6 +523,7 @@ template <int N1, int N2, bool MIXED>
 __global__ void __launch_bounds__(Shape<N1, N2>::template z_threads<MIXED>(),
                                   min_blocks(Shape<N1, N2>::template z_threads<MIXED>(), 80))
     k_fftr_zi(const Item* items, int nitems, const SysParams* sp) {
+    pdl_sync();
     using T = typename std::conditional<MIXED, float, double>::type;
     using T2 = typename C2<T>::type;
     using S = Shape<N1, N2>;
@@ -591,31 +595,36 @@ __global__ void __launch_bounds__(Shape<N1, N2>::template z_threads<MIXED>(),
 
 // One pass of the register form <N1, N2> over the items of `il`.
 template <int N1, int N2, bool MIXED>
-void launch_pass(int pass, const ItemList& il, const SysParams* sp, cudaStream_t s) {
+void launch_pass(int pass, const ItemList& il, const SysParams* sp, cudaStream_t s, bool pdl) {
     using S = Shape<N1, N2>;
     constexpr int zt = S::template z_threads<MIXED>(), ct = S::template col_threads<MIXED>();
+    auto go = [&](auto kernel, int threads) {
+        launch_k(kernel, il.grid, threads, 0, s, pdl, il.d, il.n, sp);
+    };
     switch (pass) {
-    case 0: k_fftr_zf<N1, N2, MIXED><<<il.grid, zt, 0, s>>>(il.d, il.n, sp); break;
-    case 1: k_fftr_y<N1, N2, MIXED, false><<<il.grid, ct, 0, s>>>(il.d, il.n, sp); break;
-    case 2: k_fftr_x<N1, N2, MIXED><<<il.grid, ct, 0, s>>>(il.d, il.n, sp); break;
-    case 3: k_fftr_y<N1, N2, MIXED, true><<<il.grid, ct, 0, s>>>(il.d, il.n, sp); break;
-    default: k_fftr_zi<N1, N2, MIXED><<<il.grid, zt, 0, s>>>(il.d, il.n, sp); break;
+    case 0: go(k_fftr_zf<N1, N2, MIXED>, zt); break;
+    case 1: go(k_fftr_y<N1, N2, MIXED, false>, ct); break;
+    case 2: go(k_fftr_x<N1, N2, MIXED>, ct); break;
+    case 3: go(k_fftr_y<N1, N2, MIXED, true>, ct); break;
+    default: go(k_fftr_zi<N1, N2, MIXED>, zt); break;
     }
 }
 
 #define ATVB_FFTR_CASE(i, len, a, b)                                                    \
-    case i: launch_pass<a, b, MIXED>(pass, il, sp, s); return true;
+    case i: launch_pass<a, b, MIXED>(pass, il, sp, s, pdl); return true;
 
 // The launch of form `idx` if it is in the first (second) half of the table.
 template <bool MIXED>
-bool launch_half_a(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s) {
+bool launch_half_a(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s,
+                   bool pdl) {
     switch (idx) {
         ATVB_FFTR_SIZES_A(ATVB_FFTR_CASE)
     default: return false;
     }
 }
 template <bool MIXED>
-bool launch_half_b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s) {
+bool launch_half_b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s,
+                   bool pdl) {
     switch (idx) {
         ATVB_FFTR_SIZES_B(ATVB_FFTR_CASE)
     default: return false;

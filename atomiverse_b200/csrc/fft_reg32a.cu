@@ -5,8 +5,8 @@
 namespace atvb {
 
 bool fftr_launch_32a(int pass, int idx, const ItemList& il, const SysParams* sp,
-                     cudaStream_t s) {
-    return fftr::launch_half_a<true>(pass, idx, il, sp, s);
+                     cudaStream_t s, bool pdl) {
+    return fftr::launch_half_a<true>(pass, idx, il, sp, s, pdl);
 }
 
 } // namespace atvb

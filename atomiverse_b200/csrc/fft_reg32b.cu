@@ -5,8 +5,8 @@
 namespace atvb {
 
 bool fftr_launch_32b(int pass, int idx, const ItemList& il, const SysParams* sp,
-                     cudaStream_t s) {
-    return fftr::launch_half_b<true>(pass, idx, il, sp, s);
+                     cudaStream_t s, bool pdl) {
+    return fftr::launch_half_b<true>(pass, idx, il, sp, s, pdl);
 }
 
 } // namespace atvb

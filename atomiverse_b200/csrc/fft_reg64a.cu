@@ -6,9 +6,9 @@
 
 namespace atvb {
 
-bool fftr_launch_64b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s);
-bool fftr_launch_32a(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s);
-bool fftr_launch_32b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s);
+bool fftr_launch_64b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s, bool pdl);
+bool fftr_launch_32a(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s, bool pdl);
+bool fftr_launch_32b(int pass, int idx, const ItemList& il, const SysParams* sp, cudaStream_t s, bool pdl);
 
 int fft_reg_index(int n) {
     switch (n) {
@@ -33,14 +33,14 @@ int fft_reg_lines(int idx, bool mixed) {
 int fft_reg_cols(bool mixed) { return mixed ? fftr::cols<true>() : fftr::cols<false>(); }
 
 void launch_fft_reg(int pass, int idx, bool mixed, const ItemList& il, const SysParams* sp,
-                    cudaStream_t s) {
+                    cudaStream_t s, bool pdl) {
     if (il.n == 0)
         return;
     if (mixed) {
-        if (!fftr_launch_32a(pass, idx, il, sp, s))
-            fftr_launch_32b(pass, idx, il, sp, s);
-    } else if (!fftr::launch_half_a<false>(pass, idx, il, sp, s)) {
-        fftr_launch_64b(pass, idx, il, sp, s);
+        if (!fftr_launch_32a(pass, idx, il, sp, s, pdl))
+            fftr_launch_32b(pass, idx, il, sp, s, pdl);
+    } else if (!fftr::launch_half_a<false>(pass, idx, il, sp, s, pdl)) {
+        fftr_launch_64b(pass, idx, il, sp, s, pdl);
     }
 }
 

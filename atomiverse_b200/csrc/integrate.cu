@@ -134,16 +134,143 @@ ATVB_DEV double npt_drift_atom(const SysParams& P, int i) {
     return P.mass[i] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
 }
 
+// Thermostat scalar of the initial half, neighbour decision (every / delay /
+// check), step accumulators reset, on a copy `st` of the system's state.
+// Inside the step graph (use_cond), a system that builds its list sets the
+// graph's two conditional handles (one per conditional node: the cell sort
+// and the rows), which launch the list-build kernels of this step.
+__device__ __noinline__ void sys_a_update(const SysParams& P, SysState* st,
+                                          cudaGraphConditionalHandle cond_sort,
+                                          cudaGraphConditionalHandle cond_rows, int use_cond) {
+    if (P.thermostat == kNPT || P.deform_axis >= 0) {
+        // commit the cell of this step's drift: every later kernel of the
+        // step (neighbour build, forces, PME) reads it from SysParams
+        apply_box(const_cast<SysParams&>(P), st->Lnext, true);
+        for (int d = 0; d < 3; ++d)
+            st->box[d] = st->Lnext[d];
+    }
+    st->vscale = 1.0;
+    st->nearq_n = 0; // the previous step's near-cutoff queue has been settled
+    if (P.thermostat == kNoseHoover) {
+        const double ke = fix_to_d(st->acc[kAccKEA]);
+        st->acc[kAccKEA] = 0ull;
+        st->xi += (P.dt * 0.5) * (2.0 * ke - P.n_dof_kT) / P.Q;
+        st->s_a = exp(-P.dt * 0.5 * st->xi);
+    } else {
+        st->s_a = 1.0;
+    }
+    st->ago += 1;
+    const bool disp = st->need_rebuild != 0;
+    st->need_rebuild = 0;
+    // a build the host asked for (rows widened after one was cut) comes
+    // first, whatever every/delay/check would say
+    const bool forced = st->force_build != 0;
+    st->force_build = 0;
+    const bool rebuild = forced || (st->ago >= P.nl_delay && (st->ago % P.nl_every) == 0 &&
+                                    (!P.nl_check || disp));
+    st->rebuild = rebuild ? 1 : 0;
+    if (rebuild && use_cond) {
+        cudaGraphSetConditional(cond_sort, 1u);
+        cudaGraphSetConditional(cond_rows, 1u);
+    }
+    if (rebuild) {
+        st->overflow = 0; // set again by the build if a row is cut
+        for (int d = 0; d < 3; ++d) {
+            st->Lb[d] = P.L[d];
+            st->Lb_inv[d] = 1.0 / P.L[d];
+        }
+        st->ago = 0;
+        st->rebuilds += 1;
+        st->max_nnbr = 0;
+        st->list_entries = 0ull;
+    }
+}
+
+// One thread per system, for steps whose scalar updates run as kernels of
+// their own (user components between the phases).
+__global__ void k_sys_a(const int* sys_list, int nsys, const SysParams* sp) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nsys)
+        return;
+    const SysParams& P = sp[sys_list[k]];
+    SysState* gst = P.st;
+    if (gst->halted) {
+        gst->rebuild = 0; // nothing of this system moves: no list build either
+        return;
+    }
+    SysState loc = *gst;
+    sys_a_update(P, &loc, 0, 0, 0);
+    *gst = loc;
+}
+
+// The scalar updates of a system by the block that finishes the last of its
+// atom items (counted in `ticket`): the state and the parameters are copied
+// to shared memory by all threads, the state updated there by one and copied
+// back -- a launch of its own for this one thread per system took 6 to 10 us
+// of a small system's step.
+// The ticket's acquire-release orders the item's writes (sums, status and
+// rebuild flags) before it, and the last block's reads after every ticket.
+struct ScalarShared {
+    SysState st;
+    SysParams P;
+    int last;
+};
+
+template <typename F>
+ATVB_DEV void last_item(const SysParams& P, unsigned* ticket, ScalarShared& sh, F&& update) {
+    __syncthreads(); // every thread's writes of this item come before the ticket
+    if (threadIdx.x == 0) {
+        const unsigned n = (unsigned)((P.n + kChunk - 1) / kChunk);
+        unsigned t;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                     : "=r"(t)
+                     : "l"(ticket)
+                     : "memory");
+        sh.last = t == n - 1u;
+    }
+    __syncthreads();
+    if (sh.last) {
+        constexpr int words = (int)(sizeof(SysState) / sizeof(unsigned));
+        constexpr int pwords = (int)(sizeof(SysParams) / sizeof(unsigned));
+        unsigned* g = reinterpret_cast<unsigned*>(P.st);
+        unsigned* l = reinterpret_cast<unsigned*>(&sh.st);
+        const unsigned* gp = reinterpret_cast<const unsigned*>(&P);
+        unsigned* lp = reinterpret_cast<unsigned*>(&sh.P);
+        for (int k = threadIdx.x; k < words; k += blockDim.x)
+            l[k] = __ldcg(g + k);
+        for (int k = threadIdx.x; k < pwords; k += blockDim.x)
+            lp[k] = gp[k];
+        __syncthreads();
+        // an update that may commit a cell writes SysParams itself
+        const bool cell = sh.P.thermostat == kNPT || sh.P.baro || sh.P.deform_axis >= 0;
+        if (threadIdx.x == 0)
+            update(cell ? P : sh.P, &sh.st);
+        __syncthreads();
+        for (int k = threadIdx.x; k < words; k += blockDim.x)
+            g[k] = l[k];
+        if (threadIdx.x == 0)
+            *ticket = 0u;
+    }
+}
+
 // Initial half: deferred scale, kick, drift, wrap, sorted repack,
-// displacement check, KE of the kicked velocities (for Nose-Hoover).
+// displacement check, KE of the kicked velocities (for Nose-Hoover); with
+// `fuse`, the last item of a system also runs its scalar updates.
 __global__ void __launch_bounds__(kChunk, 3)
-    k_integrate_a(const Item* items, int nitems, const SysParams* sp) {
+    k_integrate_a(const Item* items, int nitems, const SysParams* sp, int fuse,
+                  cudaGraphConditionalHandle cond_sort, cudaGraphConditionalHandle cond_rows,
+                  int use_cond) {
     __shared__ double sh[32];
+    __shared__ ScalarShared ss;
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
-        if (P.st->halted)
-            continue; // block-uniform: the item belongs to one system
+        if (P.st->halted) { // block-uniform: the item belongs to one system
+            if (fuse && item.begin == 0 && threadIdx.x == 0)
+                P.st->rebuild = 0; // nothing of it moves: no list build either
+            continue;
+        }
         const int i = item.begin + threadIdx.x;
         double ke = 0.0;
         if (i < P.n && (P.thermostat == kNPT || P.generic_drift)) {
@@ -208,74 +335,11 @@ __global__ void __launch_bounds__(kChunk, 3)
             if (threadIdx.x == 0)
                 fix_add(&P.st->acc[kAccKEA], 0.5 * kMvv2e * t);
         }
+        if (fuse)
+            last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
+                sys_a_update(Q, st, cond_sort, cond_rows, use_cond);
+            });
     }
-}
-
-// One thread per system: thermostat scalar of the initial half, neighbour
-// decision (every / delay / check), step accumulators reset.  Inside the
-// step graph (use_cond), a system that builds its list sets the graph's
-// two conditional handles (one per conditional node: the cell sort and the
-// rows), which launch the list-build kernels of this step.
-__global__ void k_sys_a(const int* sys_list, int nsys, const SysParams* sp,
-                        cudaGraphConditionalHandle cond_sort,
-                        cudaGraphConditionalHandle cond_rows, int use_cond) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsys)
-        return;
-    const SysParams& P = sp[sys_list[k]];
-    SysState* gst = P.st;
-    if (gst->halted) {
-        gst->rebuild = 0; // nothing of this system moves: no list build either
-        return;
-    }
-    // the state in local memory, written back once: each read below is then
-    // an L1 hit instead of a global round trip ordered behind the previous
-    // store (this thread is the state's only reader and writer meanwhile)
-    SysState loc = *gst;
-    SysState* st = &loc;
-    if (P.thermostat == kNPT || P.deform_axis >= 0) {
-        // commit the cell of this step's drift: every later kernel of the
-        // step (neighbour build, forces, PME) reads it from SysParams
-        apply_box(const_cast<SysParams&>(sp[sys_list[k]]), st->Lnext, true);
-        for (int d = 0; d < 3; ++d)
-            st->box[d] = st->Lnext[d];
-    }
-    st->vscale = 1.0;
-    st->nearq_n = 0; // the previous step's near-cutoff queue has been settled
-    if (P.thermostat == kNoseHoover) {
-        const double ke = fix_to_d(st->acc[kAccKEA]);
-        st->acc[kAccKEA] = 0ull;
-        st->xi += (P.dt * 0.5) * (2.0 * ke - P.n_dof_kT) / P.Q;
-        st->s_a = exp(-P.dt * 0.5 * st->xi);
-    } else {
-        st->s_a = 1.0;
-    }
-    st->ago += 1;
-    const bool disp = st->need_rebuild != 0;
-    st->need_rebuild = 0;
-    // a build the host asked for (rows widened after one was cut) comes
-    // first, whatever every/delay/check would say
-    const bool forced = st->force_build != 0;
-    st->force_build = 0;
-    const bool rebuild = forced || (st->ago >= P.nl_delay && (st->ago % P.nl_every) == 0 &&
-                                    (!P.nl_check || disp));
-    st->rebuild = rebuild ? 1 : 0;
-    if (rebuild && use_cond) {
-        cudaGraphSetConditional(cond_sort, 1u);
-        cudaGraphSetConditional(cond_rows, 1u);
-    }
-    if (rebuild) {
-        st->overflow = 0; // set again by the build if a row is cut
-        for (int d = 0; d < 3; ++d) {
-            st->Lb[d] = P.L[d];
-            st->Lb_inv[d] = 1.0 / P.L[d];
-        }
-        st->ago = 0;
-        st->rebuilds += 1;
-        st->max_nnbr = 0;
-        st->list_entries = 0ull;
-    }
-    *gst = loc;
 }
 
 // sqrt(2 kB T / (damp dt mvv2e)) / ftm2v at the setpoint of `step`: the
@@ -289,86 +353,6 @@ ATVB_DEV double lang_g2pre(const SysParams& P, long long step) {
     delta = delta < 0.0 ? 0.0 : (delta > 1.0 ? 1.0 : delta);
     const double T = __dadd_rn(P.lang_T0, __dmul_rn(delta, __dsub_rn(P.lang_T1, P.lang_T0)));
     return __ddiv_rn(__dsqrt_rn(__ddiv_rn(__dmul_rn(2.0 * kKB, T), P.lang_ddm)), kFtm2v);
-}
-
-// Final half: initial-half thermostat scale, Langevin force, kick, KE.
-__global__ void __launch_bounds__(kChunk)
-    k_integrate_b(const Item* items, int nitems, const SysParams* sp) {
-    __shared__ double sh[32];
-    __shared__ double sh3[32 * 3];
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-        const Item item = items[it];
-        const SysParams& P = sp[item.sys];
-        if (P.st->halted)
-            continue;
-        const int i = item.begin + threadIdx.x;
-        double ke = 0.0;
-        double kax[3] = {0.0, 0.0, 0.0};
-        // system fields read after the force store below, read before it
-        // (a load after a global store cannot be hoisted above it)
-        const double dtf = P.dtf, vlimit = P.vlimit, vlimit2 = P.vlimit2;
-        const int thermostat = P.thermostat;
-        if (i < P.n) {
-            const double sc = P.st->s_a;
-            const int r = P.rank[i];
-            double4 f = P.f4[r];
-            const double m = P.mass[i];
-            double v[3] = {__dmul_rn(P.vx[i], sc), __dmul_rn(P.vy[i], sc),
-                           __dmul_rn(P.vz[i], sc)};
-            if (P.has_pme) {
-                // pair + reciprocal forces; the sum is the step's force
-                const double4 g = P.fp4[r];
-                f.x = __dadd_rn(f.x, g.x);
-                f.y = __dadd_rn(f.y, g.y);
-                f.z = __dadd_rn(f.z, g.z);
-            }
-            if (P.ext_f) {
-                // the user components' forces (atvb_system_add_component)
-                f.x = __dadd_rn(f.x, P.ext_f[i]);
-                f.y = __dadd_rn(f.y, P.ext_f[P.n + i]);
-                f.z = __dadd_rn(f.z, P.ext_f[2 * P.n + i]);
-            }
-            if ((P.has_pme || P.ext_f) && thermostat != kLangevin)
-                P.f4[r] = f;
-            if (thermostat == kLangevin) {
-                const unsigned long long base =
-                    (unsigned long long)P.seed * 0x9E3779B97F4A7C15ull +
-                    (unsigned long long)P.st->step * 0xBF58476D1CE4E5B9ull;
-                GaussStream g{base + (unsigned long long)P.tag[i] *
-                                         0xD6E8FEB86659FD93ull,
-                              false, 0.0};
-                const double g1 = -m * P.lang_g1;
-                const double g2 = lang_g2pre(P, P.st->step) * sqrt(m);
-                const double rx = g.next(), ry = g.next(), rz = g.next();
-                f.x += g1 * v[0] + g2 * rx;
-                f.y += g1 * v[1] + g2 * ry;
-                f.z += g1 * v[2] + g2 * rz;
-                P.f4[r] = f;
-            }
-            const double dtfm = dtf / m;
-            v[0] = __dadd_rn(v[0], __dmul_rn(dtfm, f.x));
-            v[1] = __dadd_rn(v[1], __dmul_rn(dtfm, f.y));
-            v[2] = __dadd_rn(v[2], __dmul_rn(dtfm, f.z));
-            speed_cap(vlimit, vlimit2, v);
-            P.vx[i] = v[0];
-            P.vy[i] = v[1];
-            P.vz[i] = v[2];
-            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-            kax[0] = m * v[0] * v[0];
-            kax[1] = m * v[1] * v[1];
-            kax[2] = m * v[2] * v[2];
-        }
-        if (thermostat == kNPT) {
-            block_sum_vec<3>(kax, sh3);
-            if (threadIdx.x == 0)
-                for (int d = 0; d < 3; ++d)
-                    fix_add(&P.st->acc[kAccKEX + d], 0.5 * kMvv2e * kax[d]);
-        } else {
-            const double t = block_sum(ke, sh);
-            if (threadIdx.x == 0)
-                fix_add(&P.st->acc[kAccKEB], 0.5 * kMvv2e * t);
-        }
-    }
 }
 
 ATVB_DEV void finish_energy(const SysParams& P, SysState* st) {
@@ -409,7 +393,10 @@ ATVB_DEV void end_status(const SysParams& P, SysState* st) {
 
 ATVB_DEV void record_history(const SysParams& P, SysState* st) {
     if (P.ehist_cap > 0) {
-        const long long slot = st->step % P.ehist_cap;
+        // a 32-bit remainder while the count allows (a 64-bit one is a call)
+        const long long slot = st->step < (1ll << 31)
+                                   ? (long long)((unsigned)st->step % (unsigned)P.ehist_cap)
+                                   : st->step % P.ehist_cap;
         P.ehist[3 * slot + 0] = st->energy;
         P.ehist[3 * slot + 1] = st->kinetic;
         P.ehist[3 * slot + 2] = (double)st->step;
@@ -545,22 +532,11 @@ ATVB_DEV void npt_end_of_step(const SysParams& P, SysState* st) {
     npt_prepare(P, st, ke, vs_out);
 }
 
-// One thread per system: final-half thermostat, end-of-step scalars,
-// energy history, step counter.
-__global__ void k_sys_b(const int* sys_list, int nsys, const SysParams* sp) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsys)
-        return;
-    const SysParams& P = sp[sys_list[k]];
-    SysState* gst = P.st;
-    if (gst->halted)
-        return;
-    // the state in local memory, written back once (as in k_sys_a)
-    SysState loc = *gst;
-    SysState* st = &loc;
+// Final-half thermostat, end-of-step scalars, energy history, step counter,
+// on a copy `st` of the system's state.
+__device__ __noinline__ void sys_b_update(const SysParams& P, SysState* st) {
     if (P.thermostat == kNPT) {
         npt_end_of_step(P, st);
-        *gst = loc;
         return;
     }
     const double ke = fix_to_d(st->acc[kAccKEB]);
@@ -584,17 +560,201 @@ __global__ void k_sys_b(const int* sys_list, int nsys, const SysParams* sp) {
     else if (P.generic_drift)
         for (int d = 0; d < 3; ++d)
             st->vs[d] = st->vscale; // fixed cell: the identity drift factors stay
-    if (P.ehist_cap > 0) {
-        const long long slot = st->step % P.ehist_cap;
-        P.ehist[3 * slot + 0] = st->energy;
-        P.ehist[3 * slot + 1] = st->kinetic;
-        P.ehist[3 * slot + 2] = (double)st->step;
-    }
-    if (P.row_hint && st->rebuild) // the longest row changes only at a build
-        *(volatile int*)P.row_hint = st->max_nnbr;
-    end_status(P, st);
+    record_history(P, st);
     st->step += 1;
+}
+
+// One thread per system (see k_sys_a).
+__global__ void k_sys_b(const int* sys_list, int nsys, const SysParams* sp) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nsys)
+        return;
+    const SysParams& P = sp[sys_list[k]];
+    SysState* gst = P.st;
+    if (gst->halted)
+        return;
+    SysState loc = *gst;
+    sys_b_update(P, &loc);
     *gst = loc;
+}
+
+// Langevin friction and random force of atom i at velocity v, added to f.
+ATVB_DEV void langevin_force(const SysParams& P, int i, double m, const double v[3], double4& f) {
+    const unsigned long long base = (unsigned long long)P.seed * 0x9E3779B97F4A7C15ull +
+                                    (unsigned long long)P.st->step * 0xBF58476D1CE4E5B9ull;
+    GaussStream g{base + (unsigned long long)P.tag[i] * 0xD6E8FEB86659FD93ull, false, 0.0};
+    const double g1 = -m * P.lang_g1;
+    const double g2 = lang_g2pre(P, P.st->step) * sqrt(m);
+    const double rx = g.next(), ry = g.next(), rz = g.next();
+    f.x += g1 * v[0] + g2 * rx;
+    f.y += g1 * v[1] + g2 * ry;
+    f.z += g1 * v[2] + g2 * rz;
+}
+
+// Final half: initial-half thermostat scale, Langevin force, kick, KE; with
+// `fuse`, the last item of a system also runs its scalar updates.
+__global__ void __launch_bounds__(kChunk, 4)
+    k_integrate_b(const Item* items, int nitems, const SysParams* sp, int fuse) {
+    __shared__ double sh[32];
+    __shared__ double sh3[32 * 3];
+    __shared__ ScalarShared ss;
+    pdl_sync();
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const Item item = items[it];
+        const SysParams& P = sp[item.sys];
+        if (P.st->halted)
+            continue;
+        const int i = item.begin + threadIdx.x;
+        double ke = 0.0;
+        double kax[3] = {0.0, 0.0, 0.0};
+        // system fields read after the force store below, read before it
+        // (a load after a global store cannot be hoisted above it)
+        const double dtf = P.dtf, vlimit = P.vlimit, vlimit2 = P.vlimit2;
+        const int thermostat = P.thermostat;
+        if (i < P.n) {
+            const double sc = P.st->s_a;
+            const int r = P.rank[i];
+            double4 f = P.f4[r];
+            const double m = P.mass[i];
+            double v[3] = {__dmul_rn(P.vx[i], sc), __dmul_rn(P.vy[i], sc),
+                           __dmul_rn(P.vz[i], sc)};
+            if (P.has_pme) {
+                // pair + reciprocal forces; the sum is the step's force
+                const double4 g = P.fp4[r];
+                f.x = __dadd_rn(f.x, g.x);
+                f.y = __dadd_rn(f.y, g.y);
+                f.z = __dadd_rn(f.z, g.z);
+            }
+            if (P.ext_f) {
+                // the user components' forces (atvb_system_add_component)
+                f.x = __dadd_rn(f.x, P.ext_f[i]);
+                f.y = __dadd_rn(f.y, P.ext_f[P.n + i]);
+                f.z = __dadd_rn(f.z, P.ext_f[2 * P.n + i]);
+            }
+            if ((P.has_pme || P.ext_f) && thermostat != kLangevin)
+                P.f4[r] = f;
+            if (thermostat == kLangevin) {
+                langevin_force(P, i, m, v, f);
+                P.f4[r] = f;
+            }
+            const double dtfm = dtf / m;
+            v[0] = __dadd_rn(v[0], __dmul_rn(dtfm, f.x));
+            v[1] = __dadd_rn(v[1], __dmul_rn(dtfm, f.y));
+            v[2] = __dadd_rn(v[2], __dmul_rn(dtfm, f.z));
+            speed_cap(vlimit, vlimit2, v);
+            P.vx[i] = v[0];
+            P.vy[i] = v[1];
+            P.vz[i] = v[2];
+            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            kax[0] = m * v[0] * v[0];
+            kax[1] = m * v[1] * v[1];
+            kax[2] = m * v[2] * v[2];
+        }
+        if (thermostat == kNPT) {
+            block_sum_vec<3>(kax, sh3);
+            if (threadIdx.x == 0)
+                for (int d = 0; d < 3; ++d)
+                    fix_add(&P.st->acc[kAccKEX + d], 0.5 * kMvv2e * kax[d]);
+        } else {
+            const double t = block_sum(ke, sh);
+            if (threadIdx.x == 0)
+                fix_add(&P.st->acc[kAccKEB], 0.5 * kMvv2e * t);
+        }
+        if (fuse)
+            last_item(P, P.tickets + 1, ss,
+                      [&](const SysParams& Q, SysState* st) { sys_b_update(Q, st); });
+    }
+}
+
+// The final half of one step and the initial half of the next in one pass,
+// for engines whose systems need no system-wide sum between the two (NVE or
+// Langevin: every velocity scale is 1) and do not stop within a call: the
+// same operations per atom as k_integrate_b and k_integrate_a, so the same
+// bits, without writing and reading the velocities and forces in between
+// (204 bytes per atom instead of 296) and with one launch less per step.
+__global__ void __launch_bounds__(kChunk, 3)
+    k_integrate_ba(const Item* items, int nitems, const SysParams* sp) {
+    __shared__ double sh[32];
+    __shared__ ScalarShared ss;
+    pdl_sync();
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const Item item = items[it];
+        const SysParams& P = sp[item.sys];
+        if (P.st->halted) {
+            if (item.begin == 0 && threadIdx.x == 0)
+                P.st->rebuild = 0;
+            continue;
+        }
+        const int i = item.begin + threadIdx.x;
+        double ke = 0.0;
+        if (i < P.n) {
+            const int r = P.rank[i];
+            double4 f = P.f4[r];
+            const double m = P.mass[i];
+            const double q = P.q[i];
+            const double x0[3] = {P.x[i], P.y[i], P.z[i]};
+            const double xr[3] = {P.xr[i], P.yr[i], P.zr[i]};
+            double v[3] = {P.vx[i], P.vy[i], P.vz[i]};
+            const double L[3] = {P.L[0], P.L[1], P.L[2]};
+            const double invL[3] = {P.invL[0], P.invL[1], P.invL[2]};
+            const double dt = P.dt, skin_half2 = P.skin_half2;
+            const bool mixed = P.prec == kMixed;
+            const double fs[3] = {mixed ? P.fix_scale[0] : P.fix64_scale[0],
+                                  mixed ? P.fix_scale[1] : P.fix64_scale[1],
+                                  mixed ? P.fix_scale[2] : P.fix64_scale[2]};
+            void* const pos4 = P.pos4;
+            if (P.has_pme) {
+                const double4 g = P.fp4[r];
+                f.x = __dadd_rn(f.x, g.x);
+                f.y = __dadd_rn(f.y, g.y);
+                f.z = __dadd_rn(f.z, g.z);
+            }
+            if (P.thermostat == kLangevin)
+                langevin_force(P, i, m, v, f);
+            const double dtfm = P.dtf / m;
+            const double fa[3] = {f.x, f.y, f.z};
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                v[d] = __dadd_rn(v[d], __dmul_rn(dtfm, fa[d]));
+            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            double x[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                v[d] = __dadd_rn(v[d], __dmul_rn(dtfm, fa[d]));
+                const double xd = __dadd_rn(x0[d], __dmul_rn(dt, v[d]));
+                x[d] = __dadd_rn(xd, -__dmul_rn(L[d], floor(xd / L[d])));
+            }
+            P.vx[i] = v[0];
+            P.vy[i] = v[1];
+            P.vz[i] = v[2];
+            P.x[i] = x[0];
+            P.y[i] = x[1];
+            P.z[i] = x[2];
+            check_finite(P, x, v);
+            if (mixed) {
+                int4 p;
+                p.x = (int)pos_fix(x[0], fs[0]);
+                p.y = (int)pos_fix(x[1], fs[1]);
+                p.z = (int)pos_fix(x[2], fs[2]);
+                p.w = __float_as_int((float)q);
+                reinterpret_cast<int4*>(pos4)[r] = p;
+            } else {
+                reinterpret_cast<double4*>(pos4)[r] = pack_pos64(x, fs, q);
+            }
+            const double ddx = min_img(x[0] - xr[0], L[0], invL[0]);
+            const double ddy = min_img(x[1] - xr[1], L[1], invL[1]);
+            const double ddz = min_img(x[2] - xr[2], L[2], invL[2]);
+            if (ddx * ddx + ddy * ddy + ddz * ddz > skin_half2)
+                P.st->need_rebuild = 1;
+        }
+        const double t = block_sum(ke, sh);
+        if (threadIdx.x == 0)
+            fix_add(&P.st->acc[kAccKEB], 0.5 * kMvv2e * t);
+        last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
+            sys_b_update(Q, st);
+            sys_a_update(Q, st, 0, 0, 0);
+        });
+    }
 }
 
 // Energies of a force-only evaluation (no step, no thermostat update).
@@ -906,21 +1066,26 @@ void launch_npt_prep(const LaunchCfg& lc, cudaStream_t s) {
     k_npt_prep<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
 }
 
-void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s) {
-    k_integrate_a<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
-                                                    lc.sp);
+void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl,
+                        cudaGraphConditionalHandle cond_sort,
+                        cudaGraphConditionalHandle cond_rows, bool use_cond) {
+    launch_k(k_integrate_a, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp,
+             fuse ? 1 : 0, cond_sort, cond_rows, use_cond ? 1 : 0);
 }
-void launch_sys_a(const LaunchCfg& lc, cudaStream_t s, cudaGraphConditionalHandle cond_sort,
-                  cudaGraphConditionalHandle cond_rows, bool use_cond) {
-    k_sys_a<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp, cond_sort,
-                                                 cond_rows, use_cond ? 1 : 0);
+void launch_sys_a(const LaunchCfg& lc, cudaStream_t s) {
+    k_sys_a<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
 }
-void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s) {
-    k_integrate_b<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
-                                                    lc.sp);
+void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl) {
+    launch_k(k_integrate_b, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp,
+             fuse ? 1 : 0);
+}
+void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
+    launch_k(k_integrate_ba, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp);
 }
 void launch_sys_b(const LaunchCfg& lc, cudaStream_t s) {
     k_sys_b<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
+}
+void launch_baro(const LaunchCfg& lc, cudaStream_t s) {
     if (lc.any_baro)
         k_baro_scale<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n, lc.sp);
 }

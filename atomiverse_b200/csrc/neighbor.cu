@@ -15,9 +15,50 @@
 
 namespace atvb {
 
+// Sorted place s of atom i: the permutation, the sorted records and the
+// reference positions of the build.
+ATVB_DEV void sorted_record(const SysParams& P, int i, int s) {
+    const double x = P.x[i], y = P.y[i], z = P.z[i], q = P.q[i];
+    P.perm[s] = i;
+    P.rank[i] = s;
+    P.posd4[s] = make_double4(x, y, z, q);
+    int4 v;
+    v.x = (int)pos_fix(x, P.fix_scale[0]);
+    v.y = (int)pos_fix(y, P.fix_scale[1]);
+    v.z = (int)pos_fix(z, P.fix_scale[2]);
+    v.w = 0;
+    P.lpos[s] = v;
+    if (P.prec == kMixed) {
+        v.w = __float_as_int((float)q);
+        reinterpret_cast<int4*>(P.pos4)[s] = v;
+    } else {
+        const double xx[3] = {x, y, z};
+        reinterpret_cast<double4*>(P.pos4)[s] = pack_pos64(xx, P.fix64_scale, q);
+    }
+    if (P.ntypes)
+        P.stype[s] = (unsigned char)P.type[i];
+    P.xr[i] = x;
+    P.yr[i] = y;
+    P.zr[i] = z;
+}
+
+// Cell of atom i.
+ATVB_DEV int cell_index(const SysParams& P, int i) {
+    const double p[3] = {P.x[i], P.y[i], P.z[i]};
+    int c[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        int cd = (int)floor(p[d] * P.cs_inv[d]);
+        cd = cd < 0 ? 0 : (cd > P.nc[d] - 1 ? P.nc[d] - 1 : cd);
+        c[d] = cd;
+    }
+    return (c[0] * P.nc[1] + c[1]) * P.nc[2] + c[2];
+}
+
 // Stage 1: cell of every atom (original order) and its arrival slot.
 __global__ void k_cell_count(const Item* items, int nitems,
                              const SysParams* sp) {
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -26,15 +67,7 @@ __global__ void k_cell_count(const Item* items, int nitems,
         const int i = item.begin + threadIdx.x;
         if (i >= P.n)
             continue;
-        const double p[3] = {P.x[i], P.y[i], P.z[i]};
-        int c[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            int cd = (int)floor(p[d] * P.cs_inv[d]);
-            cd = cd < 0 ? 0 : (cd > P.nc[d] - 1 ? P.nc[d] - 1 : cd);
-            c[d] = cd;
-        }
-        const int cell = (c[0] * P.nc[1] + c[1]) * P.nc[2] + c[2];
+        const int cell = cell_index(P, i);
         P.cell_of[i] = cell;
         P.slot[i] = atomicAdd(&P.cell_count[cell], 1);
     }
@@ -47,6 +80,7 @@ __global__ void k_cell_count(const Item* items, int nitems,
 __global__ void __launch_bounds__(kChunk)
     k_cell_sums(const Item* items, int nitems, const SysParams* sp) {
     __shared__ int tot[kChunk / 32];
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -78,6 +112,7 @@ __global__ void __launch_bounds__(kChunk)
     constexpr int kPer = kScanChunk / kChunk;
     __shared__ int tot[kChunk / 32], pre[kChunk / 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -129,6 +164,7 @@ __global__ void __launch_bounds__(kChunk)
 // their cells, in arrival order.
 __global__ void k_cell_scatter(const Item* items, int nitems,
                                const SysParams* sp) {
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -151,7 +187,17 @@ __global__ void k_cell_scatter(const Item* items, int nitems,
 // order, and the atoms of it that a sphere cuts out lie close together: the
 // pair kernel's gathers then touch fewer lines.  The sorted records, the
 // permutation and the reference positions are written here too.
+ATVB_DEV int sorted_place(const int2* perm0, int a, int b, int2 me) {
+    int s = a;
+    for (int k = a; k < b; ++k) {
+        const int2 o = perm0[k];
+        s += (unsigned)o.y < (unsigned)me.y || (o.y == me.y && o.x < me.x) ? 1 : 0;
+    }
+    return s;
+}
+
 __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -163,36 +209,116 @@ __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
         const int2* __restrict__ perm0 = P.perm0;
         const int2 me = perm0[t];
         const int i = me.x;
-        const double x = P.x[i], y = P.y[i], z = P.z[i], q = P.q[i];
         const int c = P.cell_of[i];
         const int a = P.cell_start[c], b = P.cell_start[c + 1];
-        int s = a;
-        for (int k = a; k < b; ++k) {
-            const int2 o = perm0[k];
-            s += (unsigned)o.y < (unsigned)me.y || (o.y == me.y && o.x < i) ? 1 : 0;
+        const int s = sorted_place(perm0, a, b, me);
+        sorted_record(P, i, s);
+    }
+}
+
+// The whole cell sort of a small system (small_sort_fits) in one block, the
+// cell counts and the cells' atoms in shared memory: one launch instead of
+// five on every step of an engine too small for the conditional build nodes
+// (about 1 us each on the steps without a build), and on the steps with one
+// 14 us for 1,728 atoms and 23 for 4,000.  Up to 8,192 atoms: at 14,000 the
+// block took 68 us,
+// the five kernels 25.
+constexpr int kSortThreads = 1024, kSortBatch = 4;
+
+size_t small_sort_smem(int n, int ncell) {
+    return (size_t)n * sizeof(int2) + ((size_t)ncell + 1) * sizeof(int);
+}
+
+__global__ void __launch_bounds__(kSortThreads)
+    k_sort_small(const int* sys_list, const SysParams* sp) {
+    extern __shared__ int2 keys[]; // n {atom, fixed-point z}, then ncell + 1 counts
+    __shared__ int tot[kSortThreads / 32];
+    pdl_sync();
+    const SysParams& P = sp[sys_list[blockIdx.x]];
+    if (!P.st->rebuild)
+        return;
+    const int n = P.n, ncell = P.ncell, tid = threadIdx.x;
+    const int lane = tid & 31, w = tid >> 5;
+    int* cnt = reinterpret_cast<int*>(keys + n);
+    for (int c = tid; c < ncell; c += kSortThreads)
+        cnt[c] = 0;
+    __syncthreads();
+    int* const cell_of = P.cell_of;
+    int* const slot = P.slot;
+    for (int i0 = tid; i0 < n; i0 += kSortBatch * kSortThreads) {
+        int c[kSortBatch]; // loads of a batch before its stores
+#pragma unroll
+        for (int k = 0; k < kSortBatch; ++k)
+            c[k] = i0 + k * kSortThreads < n ? cell_index(P, i0 + k * kSortThreads) : 0;
+#pragma unroll
+        for (int k = 0; k < kSortBatch; ++k) {
+            const int i = i0 + k * kSortThreads;
+            if (i < n) {
+                cell_of[i] = c[k];
+                slot[i] = atomicAdd(&cnt[c[k]], 1);
+            }
         }
-        P.perm[s] = i;
-        P.rank[i] = s;
-        P.posd4[s] = make_double4(x, y, z, q);
-        int4 v;
-        v.x = (int)pos_fix(x, P.fix_scale[0]);
-        v.y = (int)pos_fix(y, P.fix_scale[1]);
-        v.z = (int)pos_fix(z, P.fix_scale[2]);
-        v.w = 0;
-        P.lpos[s] = v;
-        if (P.prec == kMixed) {
-            v.w = __float_as_int((float)q);
-            reinterpret_cast<int4*>(P.pos4)[s] = v;
+    }
+    __syncthreads();
+    // exclusive scan: each thread a run of cells, then the runs' totals
+    const int per = (ncell + kSortThreads - 1) / kSortThreads;
+    const int c0 = min(tid * per, ncell), c1 = min(c0 + per, ncell);
+    int sum = 0;
+    for (int c = c0; c < c1; ++c)
+        sum += cnt[c];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o)
+            incl += t;
+    }
+    if (lane == 31)
+        tot[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+        int t = tot[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o)
+                t += u;
         }
-        else {
-            const double xx[3] = {x, y, z};
-            reinterpret_cast<double4*>(P.pos4)[s] = pack_pos64(xx, P.fix64_scale, q);
+        tot[lane] = t;
+    }
+    __syncthreads();
+    int base = incl - sum + (w > 0 ? tot[w - 1] : 0);
+    for (int c = c0; c < c1; ++c) {
+        const int v = cnt[c];
+        cnt[c] = base;
+        P.cell_start[c] = base;
+        base += v;
+    }
+    if (tid == 0) {
+        cnt[ncell] = n;
+        P.cell_start[ncell] = n;
+    }
+    __syncthreads();
+    const double fz = P.fix_scale[2];
+    const double* const z = P.z;
+#pragma unroll 4
+    for (int i = tid; i < n; i += kSortThreads)
+        keys[cnt[cell_of[i]] + slot[i]] = make_int2(i, (int)pos_fix(z[i], fz));
+    __syncthreads();
+    for (int i0 = tid; i0 < n; i0 += kSortBatch * kSortThreads) {
+        int s[kSortBatch];
+#pragma unroll
+        for (int k = 0; k < kSortBatch; ++k) {
+            const int i = i0 + k * kSortThreads;
+            if (i < n) {
+                const int c = cell_of[i];
+                s[k] = sorted_place(keys, cnt[c], cnt[c + 1], make_int2(i, (int)pos_fix(z[i], fz)));
+            }
         }
-        if (P.ntypes)
-            P.stype[s] = (unsigned char)P.type[i];
-        P.xr[i] = x;
-        P.yr[i] = y;
-        P.zr[i] = z;
+#pragma unroll
+        for (int k = 0; k < kSortBatch; ++k)
+            if (i0 + k * kSortThreads < n)
+                sorted_record(P, i0 + k * kSortThreads, s[k]);
     }
 }
 
@@ -521,6 +647,7 @@ __global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
         }
         __syncthreads();
     };
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -559,27 +686,41 @@ __global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
         flush();
 }
 
+bool small_sort_fits(int n, int ncell) { return n <= kSortSmallAtoms && ncell <= kSortSmallCells; }
+
+void sort_smem_optin() {
+    cuda_check(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)small_sort_smem(kSortSmallAtoms, kSortSmallCells)),
+               "shared memory of k_sort_small");
+}
+
 // Binning and the sorted repack: after these the sorted positions (pos4)
 // that the PME chain reads are final, so that chain may start beside the
 // list build.
-void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s) {
-    k_cell_count<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
-                                                   lc.sp);
-    k_cell_sums<<<lc.scan.grid, kChunk, 0, s>>>(lc.scan.d, lc.scan.n, lc.sp);
-    k_cell_scan<<<lc.scan.grid, kChunk, 0, s>>>(lc.scan.d, lc.scan.n, lc.sp);
-    k_cell_scatter<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n,
-                                                     lc.sp);
-    k_permute<<<lc.atoms.grid, kChunk, 0, s>>>(lc.atoms.d, lc.atoms.n, lc.sp);
+void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
+    if (lc.nsmall) {
+        launch_k(k_sort_small, lc.nsmall, kSortThreads, lc.small_smem, s, pdl, lc.small_list,
+                 lc.sp);
+        pdl = lc.pdl;
+    }
+    if (lc.sort_atoms.n) {
+        const ItemList &A = lc.sort_atoms, &S = lc.scan;
+        launch_k(k_cell_count, A.grid, kChunk, 0, s, pdl, A.d, A.n, lc.sp);
+        launch_k(k_cell_sums, S.grid, kChunk, 0, s, lc.pdl, S.d, S.n, lc.sp);
+        launch_k(k_cell_scan, S.grid, kChunk, 0, s, lc.pdl, S.d, S.n, lc.sp);
+        launch_k(k_cell_scatter, A.grid, kChunk, 0, s, lc.pdl, A.d, A.n, lc.sp);
+        launch_k(k_permute, A.grid, kChunk, 0, s, lc.pdl, A.d, A.n, lc.sp);
+    }
 }
 
-void launch_build_list(const LaunchCfg& lc, cudaStream_t s) {
-    k_build_list<<<lc.list.grid, 32 * kListChunk, 0, s>>>(lc.list.d, lc.list.n, lc.sp,
-                                                           lc.list_split_log2);
+void launch_build_list(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
+    launch_k(k_build_list, lc.list.grid, 32 * kListChunk, 0, s, pdl, lc.list.d, lc.list.n, lc.sp,
+             lc.list_split_log2);
 }
 
 void launch_rebuild(const LaunchCfg& lc, cudaStream_t s) {
-    launch_sort_cells(lc, s);
-    launch_build_list(lc, s);
+    launch_sort_cells(lc, s, false);
+    launch_build_list(lc, s, false);
 }
 
 } // namespace atvb

@@ -298,6 +298,7 @@ template <bool MIXED, int G>
 __global__ void __launch_bounds__(256, MIXED ? 3 : 2)
     k_pair(const Item* items, int nitems, const SysParams* sp) {
     __shared__ double sh[32 * 8];
+    pdl_sync();
     const int g = threadIdx.x % G;
     const int a_off = threadIdx.x / G;
     PairAcc acc;
@@ -395,6 +396,7 @@ ATVB_DEV void fix_share(const SysParams& P, int s, int code, int lane) {
 
 __global__ void __launch_bounds__(256)
     k_pair_fix(const int* sys_list, int nsys, const SysParams* sp) {
+    pdl_sync();
     const SysParams& P = sp[sys_list[blockIdx.x / kFixBlocks]];
     if (P.prec != kMixed || !P.has_lj || P.general || P.nearq == nullptr ||
         !(P.mix_band_lj > 0.0))
@@ -420,32 +422,26 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-template <bool MIXED>
-static void launch_pair_prec(const LaunchCfg& lc, cudaStream_t s) {
-    const ItemList* L = lc.pair[MIXED ? 1 : 0];
-    if (L[0].n)
-        k_pair<MIXED, 1><<<L[0].grid, kPairBlock, 0, s>>>(L[0].d, L[0].n, lc.sp);
-    if (L[1].n)
-        k_pair<MIXED, 2><<<L[1].grid, kPairBlock, 0, s>>>(L[1].d, L[1].n, lc.sp);
-    if (L[2].n)
-        k_pair<MIXED, 4><<<L[2].grid, kPairBlock, 0, s>>>(L[2].d, L[2].n, lc.sp);
-    if (L[3].n)
-        k_pair<MIXED, 8><<<L[3].grid, kPairBlock, 0, s>>>(L[3].d, L[3].n, lc.sp);
-    if (L[4].n)
-        k_pair<MIXED, 16><<<L[4].grid, kPairBlock, 0, s>>>(L[4].d, L[4].n, lc.sp);
-    if (L[5].n)
-        k_pair<MIXED, 32><<<L[5].grid, kPairBlock, 0, s>>>(L[5].d, L[5].n, lc.sp);
+template <bool MIXED, int C>
+static void launch_pair_class(const LaunchCfg& lc, cudaStream_t s, bool& pdl) {
+    const ItemList& L = lc.pair[MIXED ? 1 : 0][C];
+    if (L.n) {
+        launch_k(k_pair<MIXED, 1 << C>, L.grid, kPairBlock, 0, s, pdl, L.d, L.n, lc.sp);
+        pdl = lc.pdl;
+    }
+    if constexpr (C + 1 < kLaneClasses)
+        launch_pair_class<MIXED, C + 1>(lc, s, pdl);
 }
 
-void launch_pair(const LaunchCfg& lc, cudaStream_t s) {
-    launch_pair_prec<false>(lc, s);
-    launch_pair_prec<true>(lc, s);
-    launch_pair_general(lc, s);
+void launch_pair(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
+    launch_pair_class<false, 0>(lc, s, pdl);
+    launch_pair_class<true, 0>(lc, s, pdl);
+    launch_pair_general(lc, s, pdl);
 }
 
 void launch_pair_fix(const LaunchCfg& lc, cudaStream_t s) {
     if (lc.any_near && lc.nsys > 0)
-        k_pair_fix<<<lc.nsys * kFixBlocks, 256, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
+        launch_k(k_pair_fix, lc.nsys * kFixBlocks, 256, 0, s, lc.pdl, lc.sys_list, lc.nsys, lc.sp);
 }
 
 } // namespace atvb

@@ -169,6 +169,7 @@ template <bool MIXED>
 __global__ void __launch_bounds__(256)
     k_pair_general(const Item* items, int nitems, const SysParams* sp) {
     __shared__ double sh[32 * 8];
+    pdl_sync();
     const int g = threadIdx.x % kGenLanes;
     const int a_off = threadIdx.x / kGenLanes;
     PairAcc acc;
@@ -197,13 +198,14 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-void launch_pair_general(const LaunchCfg& lc, cudaStream_t s) {
-    if (lc.pair_gen[0].n)
-        k_pair_general<false><<<lc.pair_gen[0].grid, 256, 0, s>>>(lc.pair_gen[0].d,
-                                                                  lc.pair_gen[0].n, lc.sp);
-    if (lc.pair_gen[1].n)
-        k_pair_general<true><<<lc.pair_gen[1].grid, 256, 0, s>>>(lc.pair_gen[1].d,
-                                                                 lc.pair_gen[1].n, lc.sp);
+void launch_pair_general(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
+    const ItemList *D = &lc.pair_gen[0], *M = &lc.pair_gen[1];
+    if (D->n) {
+        launch_k(k_pair_general<false>, D->grid, 256, 0, s, pdl, D->d, D->n, lc.sp);
+        pdl = lc.pdl;
+    }
+    if (M->n)
+        launch_k(k_pair_general<true>, M->grid, 256, 0, s, pdl, M->d, M->n, lc.sp);
 }
 
 } // namespace atvb

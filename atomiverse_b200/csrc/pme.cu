@@ -148,6 +148,7 @@ template <bool MIXED, int N>
 __global__ void __launch_bounds__(kChunk)
     k_pme_spread(const Item* items, int nitems, const SysParams* sp) {
     using T = typename std::conditional<MIXED, float, double>::type;
+    pdl_sync();
     const AtomLanes<N> L;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
@@ -197,6 +198,7 @@ template <bool MIXED, int N>
 __global__ void __launch_bounds__(256)
     k_pme_gather(const Item* items, int nitems, const SysParams* sp) {
     using T = typename std::conditional<MIXED, float, double>::type;
+    pdl_sync();
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
@@ -263,14 +265,16 @@ static void spread_order(const LaunchCfg& lc, cudaStream_t s) {
 template <bool MIXED>
 static void gather_order(const LaunchCfg& lc, cudaStream_t s) {
     const ItemList& il = lc.pme_atoms;
-    constexpr int T = kChunk;
+    auto go = [&](auto kernel) {
+        launch_k(kernel, il.grid, kChunk, 0, s, lc.pdl, il.d, il.n, lc.sp);
+    };
     switch (lc.pme_order) {
-    case 3: k_pme_gather<MIXED, 3><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
-    case 4: k_pme_gather<MIXED, 4><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
-    case 5: k_pme_gather<MIXED, 5><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
-    case 6: k_pme_gather<MIXED, 6><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
-    case 7: k_pme_gather<MIXED, 7><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
-    default: k_pme_gather<MIXED, 8><<<il.grid, T, 0, s>>>(il.d, il.n, lc.sp); break;
+    case 3: go(k_pme_gather<MIXED, 3>); break;
+    case 4: go(k_pme_gather<MIXED, 4>); break;
+    case 5: go(k_pme_gather<MIXED, 5>); break;
+    case 6: go(k_pme_gather<MIXED, 6>); break;
+    case 7: go(k_pme_gather<MIXED, 7>); break;
+    default: go(k_pme_gather<MIXED, 8>); break;
     }
 }
 
