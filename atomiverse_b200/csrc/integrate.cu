@@ -80,6 +80,23 @@ ATVB_DEV void check_finite(const SysParams& P, const double x[3], const double v
         atomicOr(&P.st->status, kStatusNonFinite);
 }
 
+// m v^2, and the squared minimum-image displacement from xr: explicit
+// operations, so that the kernels that share them round alike.
+ATVB_DEV double mv2(double m, const double v[3]) {
+    return m * fma(v[2], v[2], fma(v[1], v[1], v[0] * v[0]));
+}
+ATVB_DEV double moved2(const double x[3], const double xr[3], const double L[3],
+                       const double invL[3]) {
+    double d2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double dx = x[d] - xr[d];
+        const double m = fma(-L[d], rint(dx * invL[d]), dx);
+        d2 = fma(m, m, d2);
+    }
+    return d2;
+}
+
 // MTK NPT initial half for atom i (nose_hoover_npt.cpp:812-850 P2-P6): the
 // pending per-axis velocity scale (end-of-step chain and barostat factors of
 // the previous step, initial-half ones of this step), the force kick, the
@@ -323,12 +340,9 @@ __global__ void __launch_bounds__(kChunk, 3)
                 reinterpret_cast<double4*>(pos4)[r] = pack_pos64(x, fs, q);
             }
             // cell_list.cpp:355-392 with min-image displacement
-            const double ddx = min_img(x[0] - xr[0], L[0], invL[0]);
-            const double ddy = min_img(x[1] - xr[1], L[1], invL[1]);
-            const double ddz = min_img(x[2] - xr[2], L[2], invL[2]);
-            if (ddx * ddx + ddy * ddy + ddz * ddz > skin_half2)
+            if (moved2(x, xr, L, invL) > skin_half2)
                 P.st->need_rebuild = 1;
-            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            ke = mv2(m, v);
         }
         if (P.thermostat == kNoseHoover) {
             const double t = block_sum(ke, sh);
@@ -583,12 +597,13 @@ ATVB_DEV void langevin_force(const SysParams& P, int i, double m, const double v
     const unsigned long long base = (unsigned long long)P.seed * 0x9E3779B97F4A7C15ull +
                                     (unsigned long long)P.st->step * 0xBF58476D1CE4E5B9ull;
     GaussStream g{base + (unsigned long long)P.tag[i] * 0xD6E8FEB86659FD93ull, false, 0.0};
-    const double g1 = -m * P.lang_g1;
-    const double g2 = lang_g2pre(P, P.st->step) * sqrt(m);
+    const double g1 = __dmul_rn(-m, P.lang_g1);
+    const double g2 = __dmul_rn(lang_g2pre(P, P.st->step), sqrt(m));
     const double rx = g.next(), ry = g.next(), rz = g.next();
-    f.x += g1 * v[0] + g2 * rx;
-    f.y += g1 * v[1] + g2 * ry;
-    f.z += g1 * v[2] + g2 * rz;
+    // every operation rounded on its own: the same bits wherever this is inlined
+    f.x = __dadd_rn(f.x, __dadd_rn(__dmul_rn(g1, v[0]), __dmul_rn(g2, rx)));
+    f.y = __dadd_rn(f.y, __dadd_rn(__dmul_rn(g1, v[1]), __dmul_rn(g2, ry)));
+    f.z = __dadd_rn(f.z, __dadd_rn(__dmul_rn(g1, v[2]), __dmul_rn(g2, rz)));
 }
 
 // Final half: initial-half thermostat scale, Langevin force, kick, KE; with
@@ -645,7 +660,7 @@ __global__ void __launch_bounds__(kChunk, 4)
             P.vx[i] = v[0];
             P.vy[i] = v[1];
             P.vz[i] = v[2];
-            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            ke = mv2(m, v);
             kax[0] = m * v[0] * v[0];
             kax[1] = m * v[1] * v[1];
             kax[2] = m * v[2] * v[2];
@@ -716,7 +731,7 @@ __global__ void __launch_bounds__(kChunk, 3)
 #pragma unroll
             for (int d = 0; d < 3; ++d)
                 v[d] = __dadd_rn(v[d], __dmul_rn(dtfm, fa[d]));
-            ke = m * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            ke = mv2(m, v);
             double x[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
@@ -741,10 +756,7 @@ __global__ void __launch_bounds__(kChunk, 3)
             } else {
                 reinterpret_cast<double4*>(pos4)[r] = pack_pos64(x, fs, q);
             }
-            const double ddx = min_img(x[0] - xr[0], L[0], invL[0]);
-            const double ddy = min_img(x[1] - xr[1], L[1], invL[1]);
-            const double ddz = min_img(x[2] - xr[2], L[2], invL[2]);
-            if (ddx * ddx + ddy * ddy + ddz * ddz > skin_half2)
+            if (moved2(x, xr, L, invL) > skin_half2)
                 P.st->need_rebuild = 1;
         }
         const double t = block_sum(ke, sh);
