@@ -280,7 +280,7 @@ class System:
         """Frame and scalars.  A sticky status bit (wrong or non-finite
         physics in some step) raises PhysicsError unless check=False; its
         `result` carries the (frame, scalars) anyway."""
-        out = {k: np.zeros(self.n) for k in keys}
+        out = {k: np.empty(self.n) for k in keys}
         v, keep = _soa(out, self.n, writable=True)
         s = Scalars()
         rc = self.lib.atvb_system_download(self._h, C.byref(v), C.byref(s))
@@ -425,7 +425,7 @@ class Batch:
         check(self.lib.atvb_batch_step(self._h, int(n)))
 
     def download(self, k: int, keys=FRAME_KEYS, check: bool = True) -> tuple[dict, dict]:
-        out = {key: np.zeros(self.sizes[k]) for key in keys}
+        out = {key: np.empty(self.sizes[k]) for key in keys}
         v, keep = _soa(out, self.sizes[k], writable=True)
         s = Scalars()
         rc = self.lib.atvb_batch_download(self._h, int(k), C.byref(v), C.byref(s))
@@ -508,7 +508,7 @@ class Server:
 
     def collect(self, rid: int) -> tuple[dict, dict]:
         n = self.sizes[rid]
-        out = {k: np.zeros(n) for k in FRAME_KEYS[:9]}
+        out = {k: np.empty(n) for k in FRAME_KEYS[:9]}
         v, keep = _soa(out, n, writable=True)
         r = _abi.RequestResult()
         check(self.lib.atvb_server_collect(self._h, int(rid), C.byref(v), C.byref(r)))

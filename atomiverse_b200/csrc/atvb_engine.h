@@ -78,6 +78,8 @@ class Slot {
     bool special_set = false;
     double sp_lj[3] = {1, 1, 1}, sp_coul[3] = {1, 1, 1};
     std::vector<long long> bond_a, bond_b;
+    std::vector<int> table_types;         // types the device table was built for
+    std::vector<long long> special_tags;  // tags the partner lists were built for
     void build_specials(const std::vector<long long>& tags, cudaStream_t stream);
 
     void* dalloc(size_t b);
@@ -97,6 +99,36 @@ class Slot {
     DevMem mem_;
     std::vector<void*> allocs;
     void* nbr_alloc = nullptr;
+};
+
+// One array moved between the host and the device.
+struct Xfer {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+
+// Pinned staging between pageable host arrays and the device: kPiece bytes,
+// two per worker, allocated on the first large call and kept by the engine.
+class HostStage {
+  public:
+    explicit HostStage(int device) : device_(device) {}
+    ~HostStage();
+    // device -> host, after the work already on `stream`; complete on return
+    void fetch(const std::vector<Xfer>& list, cudaStream_t stream);
+    // host -> device in stream order; the host arrays are free on return
+    void put(const std::vector<Xfer>& list, cudaStream_t stream);
+
+  private:
+    static constexpr size_t kPiece = size_t(256) << 10;
+    static constexpr size_t kStagedFrom = size_t(8) << 20; // bytes of a call
+    static constexpr int kMaxWorkers = 4;
+    void ready();
+    void run(const std::vector<Xfer>& list, cudaStream_t stream, bool out);
+    int device_;
+    int workers_ = 1;
+    char* buf_ = nullptr;
+    cudaEvent_t ev_[2 * kMaxWorkers] = {};
 };
 
 // A user component's callbacks at one phase (atvb_system_add_component).
@@ -205,6 +237,7 @@ class Engine {
     int device_ = 0;
     cudaStream_t stream_ = nullptr;
     DevMem mem_;
+    std::unique_ptr<HostStage> stage_;
     cudaStream_t pme_stream_ = nullptr; // the PME chain beside the pair kernel
     // the list build as conditional nodes of the step graph: the handle of
     // the graph being captured and the stream their bodies are captured on

@@ -17,6 +17,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -244,6 +245,122 @@ size_t estimate_bytes(const atvb_system_desc& d) {
         b += (K0 + K1 + K2) * 2 * rs; // roots of unity of the transforms
     }
     return b;
+}
+
+// ---------------------------------------------------------- HostStage
+
+HostStage::~HostStage() {
+    for (cudaEvent_t e : ev_)
+        if (e)
+            cudaEventDestroy(e);
+    if (buf_)
+        cudaFreeHost(buf_);
+}
+
+void HostStage::ready() {
+    if (buf_)
+        return;
+    const unsigned hw = std::thread::hardware_concurrency();
+    workers_ = (int)std::min<unsigned>(kMaxWorkers, std::max(1u, hw / 2));
+    for (int k = 0; k < 2 * workers_; ++k)
+        if (!ev_[k])
+            CK(cudaEventCreateWithFlags(&ev_[k], cudaEventDisableTiming));
+    void* p = nullptr;
+    CK(cudaHostAlloc(&p, 2 * kMaxWorkers * kPiece, cudaHostAllocDefault));
+    buf_ = (char*)p;
+}
+
+// The arrays in pieces of kPiece bytes; worker w moves pieces w, w + W, ...
+// through its two buffers, copying one on the host while the other is on its
+// way.  A copy straight from or to pageable memory goes through the driver's
+// own staging on the calling thread alone: the nine arrays of 1,000,188 atoms
+// (72 MB) took 9 to 21 ms to read, 3.5 to 6.4 ms through here.  The pinned
+// buffer costs 2 to 3 ms once, so a call below kStagedFrom bytes stays plain.
+void HostStage::run(const std::vector<Xfer>& list, cudaStream_t stream, bool out) {
+    struct Piece {
+        char* host;
+        char* dev;
+        size_t bytes;
+    };
+    std::vector<Piece> piece;
+    for (const Xfer& x : list)
+        for (size_t o = 0; o < x.bytes; o += kPiece)
+            piece.push_back({(char*)x.host + o, (char*)x.dev + o, std::min(kPiece, x.bytes - o)});
+    const int W = (int)std::min<size_t>(workers_, (piece.size() + 3) / 4);
+    cudaError_t err[kMaxWorkers] = {};
+    auto work = [&](int w) {
+        cudaError_t& e = err[w];
+        e = cudaSetDevice(device_);
+        const Piece* held[2] = {nullptr, nullptr}; // pieces in flight
+        int b = 0;
+        // one more round than pieces per buffer, to drain both
+        for (size_t k = w; e == cudaSuccess; k += W, b ^= 1) {
+            const int slot = 2 * w + b;
+            char* s = buf_ + (size_t)slot * kPiece;
+            if (held[b]) {
+                e = cudaEventSynchronize(ev_[slot]);
+                if (e == cudaSuccess && out)
+                    std::memcpy(held[b]->host, s, held[b]->bytes);
+                held[b] = nullptr;
+            } else if (k >= piece.size()) {
+                if (!held[b ^ 1])
+                    break;
+                continue;
+            }
+            if (e != cudaSuccess || k >= piece.size())
+                continue;
+            const Piece& p = piece[k];
+            if (!out)
+                std::memcpy(s, p.host, p.bytes);
+            e = out ? cudaMemcpyAsync(s, p.dev, p.bytes, cudaMemcpyDeviceToHost, stream)
+                    : cudaMemcpyAsync(p.dev, s, p.bytes, cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess)
+                e = cudaEventRecord(ev_[slot], stream);
+            held[b] = &p;
+        }
+    };
+    std::vector<std::thread> team;
+    team.reserve(W);
+    for (int w = 1; w < W; ++w) {
+        try {
+            team.emplace_back(work, w);
+        } catch (...) { // no thread to be had: this one does its share
+            work(w);
+        }
+    }
+    work(0);
+    for (std::thread& t : team)
+        t.join();
+    for (cudaError_t e : err)
+        cuda_check(e, "staged copy");
+}
+
+void HostStage::fetch(const std::vector<Xfer>& list, cudaStream_t stream) {
+    size_t total = 0;
+    for (const Xfer& x : list)
+        total += x.bytes;
+    if (total >= kStagedFrom) {
+        ready();
+        run(list, stream, true);
+        return;
+    }
+    for (const Xfer& x : list)
+        CK(cudaMemcpyAsync(x.host, x.dev, x.bytes, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+}
+
+void HostStage::put(const std::vector<Xfer>& list, cudaStream_t stream) {
+    size_t total = 0;
+    for (const Xfer& x : list)
+        total += x.bytes;
+    if (total >= kStagedFrom) {
+        ready();
+        run(list, stream, false);
+        return;
+    }
+    for (const Xfer& x : list)
+        CK(cudaMemcpyAsync(x.dev, x.host, x.bytes, cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream)); // the host arrays are free on return
 }
 
 // --------------------------------------------------------------- Slot
@@ -646,6 +763,7 @@ Engine::Engine(int device) : device_(device) {
     // the FFT blocks' line buffers live in dynamic shared memory above 48 KB
     fft_smem_optin(kFftSmem + 1024);
     sort_smem_optin();
+    stage_ = std::make_unique<HostStage>(device);
 }
 
 Engine::~Engine() {
@@ -2044,6 +2162,10 @@ void Engine::set_lj_types(int id, int ncoef, const int32_t* ti, const int32_t* t
 // interact (eps = 0), so a type with no coefficient has no LJ site; every
 // type pair is shifted at the common cutoff.
 void Slot::build_lj_tables(const std::vector<int>& types, cudaStream_t stream) {
+    // the same types again (new coordinates of the same atoms): the table and
+    // the per-atom types on the device stand
+    if (hp.type && types == table_types)
+        return;
     int nt = ntypes;
     for (int t : types) {
         if (t < 0 || t > 254)
@@ -2087,6 +2209,7 @@ void Slot::build_lj_tables(const std::vector<int>& types, cudaStream_t stream) {
     double* dt = (double*)dalloc(tab.size() * sizeof(double));
     float* dtf = (float*)dalloc(tabf.size() * sizeof(float));
     int* dtype = (int*)dalloc((size_t)hp.n * sizeof(int));
+    unsigned char* dstype = (unsigned char*)dalloc((size_t)hp.n);
     CK(cudaMemcpyAsync(dt, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice,
                        stream));
     CK(cudaMemcpyAsync(dtf, tabf.data(), tabf.size() * sizeof(float), cudaMemcpyHostToDevice,
@@ -2094,11 +2217,15 @@ void Slot::build_lj_tables(const std::vector<int>& types, cudaStream_t stream) {
     CK(cudaMemcpyAsync(dtype, types.data(), (size_t)hp.n * sizeof(int), cudaMemcpyHostToDevice,
                        stream));
     CK(cudaStreamSynchronize(stream));
+    for (const void* p : {(const void*)hp.lj_tab, (const void*)hp.lj_tabf,
+                          (const void*)hp.type, (const void*)hp.stype})
+        free_alloc(const_cast<void*>(p)); // those of an earlier upload
     hp.lj_tab = dt;
     hp.lj_tabf = dtf;
     hp.type = dtype;
-    hp.stype = (unsigned char*)dalloc((size_t)hp.n);
+    hp.stype = dstype;
     hp.ntypes = nt;
+    table_types = types;
 }
 
 // PairLJCut / CoulLong set_special_bonds(s12, s13, s14) with the bond
@@ -2126,6 +2253,10 @@ void Engine::set_special_bonds(int id, const double lj[3], const double coul[3],
 }
 
 void Slot::build_specials(const std::vector<long long>& tags, cudaStream_t stream) {
+    // the same tags again: the partner lists on the device stand (the bonds
+    // and scales are fixed by the first upload)
+    if (hp.has_special && tags == special_tags)
+        return;
     const int n = hp.n;
     std::unordered_map<long long, int> idx;
     idx.reserve((size_t)n * 2);
@@ -2181,6 +2312,9 @@ void Slot::build_specials(const std::vector<long long>& tags, cudaStream_t strea
         CK(cudaMemcpyAsync(d_c, cls.data(), cls.size(), cudaMemcpyHostToDevice, stream));
     }
     CK(cudaStreamSynchronize(stream));
+    for (const void* p :
+         {(const void*)hp.sp_first, (const void*)hp.sp_j, (const void*)hp.sp_cls})
+        free_alloc(const_cast<void*>(p)); // those of an earlier upload
     hp.sp_first = d_first;
     hp.sp_j = d_j;
     hp.sp_cls = d_c;
@@ -2190,6 +2324,7 @@ void Slot::build_specials(const std::vector<long long>& tags, cudaStream_t strea
         hp.sp_lj[k + 1] = sp_lj[k];
         hp.sp_coul[k + 1] = sp_coul[k];
     }
+    special_tags = tags;
 }
 
 void Engine::upload(int id, const atvb_soa_view& f) {
@@ -2197,19 +2332,16 @@ void Engine::upload(int id, const atvb_soa_view& f) {
     Slot* s = slot(id);
     const int n = s->hp.n;
     const size_t b = sizeof(double) * n;
-    std::vector<double> tmp;
-    auto put = [&](double* dst, const double* src, double fill) {
-        if (src) {
-            CK(cudaMemcpyAsync(dst, src, b, cudaMemcpyHostToDevice, stream_));
-        } else {
-            tmp.assign(n, fill);
-            CK(cudaMemcpyAsync(dst, tmp.data(), b, cudaMemcpyHostToDevice,
-                               stream_));
-            CK(cudaStreamSynchronize(stream_));
-        }
-    };
     if (!f.x || !f.y || !f.z)
         throw Error(ATVB_ERR_INVALID, "upload needs positions");
+    std::vector<Xfer> in;
+    std::vector<double> zeros, ones;
+    auto put = [&](double* dst, const double* src, double fill) {
+        std::vector<double>& v = fill == 0.0 ? zeros : ones;
+        if (!src && v.empty())
+            v.assign(n, fill);
+        in.push_back({const_cast<double*>(src ? src : v.data()), dst, b});
+    };
     put(s->hp.x, f.x, 0.0);
     put(s->hp.y, f.y, 0.0);
     put(s->hp.z, f.z, 0.0);
@@ -2228,8 +2360,8 @@ void Engine::upload(int id, const atvb_soa_view& f) {
     std::vector<long long> tag(n);
     for (int i = 0; i < n; ++i)
         tag[i] = f.tag ? f.tag[i] : (long long)(i + 1);
-    CK(cudaMemcpyAsync(s->hp.tag, tag.data(), 8 * n, cudaMemcpyHostToDevice,
-                       stream_));
+    in.push_back({tag.data(), s->hp.tag, (size_t)n * sizeof(long long)});
+    stage_->put(in, stream_);
     if (s->ntypes > 0) {
         std::vector<int> ty(n, 0);
         if (f.type)
@@ -2288,10 +2420,13 @@ void Engine::upload(int id, const atvb_soa_view& f) {
     CK(cudaStreamSynchronize(stream_));
     if (row_hint_host_ && id < sp_cap_)
         ((volatile int*)row_hint_host_)[sp_cap_ + id] = 0; // a fresh state: no status
+    // the work lists of a system that was here before still hold
+    if (!s->uploaded)
+        dirty_ = true;
     s->uploaded = true;
     s->snap_read = 0; // the published snapshot count restarts with the state
-    dirty_ = true;
-    build_lists();
+    if (dirty_)
+        build_lists();
     // wrap, first neighbour build, uploaded forces into sorted order, KE --
     // touching only this system
     const LaunchCfg one = restricted_cfg(id);
@@ -2309,7 +2444,8 @@ void Engine::upload(int id, const atvb_soa_view& f) {
     SysState st;
     CK(cudaMemcpy(&st, s->hp.st, sizeof(st), cudaMemcpyDeviceToHost));
     s->mean_row = st.max_nnbr;
-    dirty_ = true; // lane choice may change with the measured row length
+    if (lanes_for(*s) != s->lanes)
+        dirty_ = true; // the lane choice follows the measured row length
 }
 
 void Engine::scalars(int id, atvb_scalars* out) {
@@ -2355,49 +2491,35 @@ void Engine::download(int id, atvb_soa_view* f, atvb_scalars* sc) {
     ensure_ready();
     const LaunchCfg one = restricted_cfg(id);
     if (f) {
-        if (f->x)
-            CK(cudaMemcpyAsync(f->x, s->hp.x, b, cudaMemcpyDeviceToHost, stream_));
-        if (f->y)
-            CK(cudaMemcpyAsync(f->y, s->hp.y, b, cudaMemcpyDeviceToHost, stream_));
-        if (f->z)
-            CK(cudaMemcpyAsync(f->z, s->hp.z, b, cudaMemcpyDeviceToHost, stream_));
-        if (f->mass)
-            CK(cudaMemcpyAsync(f->mass, s->hp.mass, b, cudaMemcpyDeviceToHost,
-                               stream_));
-        if (f->charge)
-            CK(cudaMemcpyAsync(f->charge, s->hp.q, b, cudaMemcpyDeviceToHost,
-                               stream_));
+        const SysParams& P = s->hp;
+        std::vector<Xfer> get;
+        auto add = [&](double* host, double* dev) {
+            if (host)
+                get.push_back({host, dev, b});
+        };
+        add(f->x, P.x);
+        add(f->y, P.y);
+        add(f->z, P.z);
+        add(f->mass, P.mass);
+        add(f->charge, P.q);
+        if (f->tag)
+            get.push_back({f->tag, P.tag, (size_t)n * sizeof(int64_t)});
         if (f->fx || f->fy || f->fz) {
             launch_state_out(one, 0, stream_);
-            if (f->fx)
-                CK(cudaMemcpyAsync(f->fx, s->hp.sx, b, cudaMemcpyDeviceToHost,
-                                   stream_));
-            if (f->fy)
-                CK(cudaMemcpyAsync(f->fy, s->hp.sy, b, cudaMemcpyDeviceToHost,
-                                   stream_));
-            if (f->fz)
-                CK(cudaMemcpyAsync(f->fz, s->hp.sz, b, cudaMemcpyDeviceToHost,
-                                   stream_));
+            add(f->fx, P.sx);
+            add(f->fy, P.sy);
+            add(f->fz, P.sz);
         }
-        if (f->vx || f->vy || f->vz) {
+        const bool vel = f->vx || f->vy || f->vz;
+        if (!get.empty())
+            stage_->fetch(get, stream_);
+        if (vel) { // through the same device arrays as the forces
+            get.clear();
             launch_state_out(one, 1, stream_);
-            if (f->vx)
-                CK(cudaMemcpyAsync(f->vx, s->hp.sx, b, cudaMemcpyDeviceToHost,
-                                   stream_));
-            if (f->vy)
-                CK(cudaMemcpyAsync(f->vy, s->hp.sy, b, cudaMemcpyDeviceToHost,
-                                   stream_));
-            if (f->vz)
-                CK(cudaMemcpyAsync(f->vz, s->hp.sz, b, cudaMemcpyDeviceToHost,
-                                   stream_));
-        }
-        if (f->tag) {
-            std::vector<long long> t(n);
-            CK(cudaMemcpyAsync(t.data(), s->hp.tag, 8 * n,
-                               cudaMemcpyDeviceToHost, stream_));
-            CK(cudaStreamSynchronize(stream_));
-            for (int i = 0; i < n; ++i)
-                f->tag[i] = t[i];
+            add(f->vx, P.sx);
+            add(f->vy, P.sy);
+            add(f->vz, P.sz);
+            stage_->fetch(get, stream_);
         }
     }
     CK(cudaStreamSynchronize(stream_));
