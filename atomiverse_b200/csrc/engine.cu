@@ -950,16 +950,19 @@ static ItemList make_list(std::vector<void*>& allocs, const std::vector<Item>& v
 // Lanes per atom for one system, from that system alone: at least 4 (the
 // lanes of an atom read consecutive row entries, so a warp's row loads
 // coalesce; measured on 1M LJ atoms: 4 lanes 27 % (FP64) and 35 % (mixed)
-// faster than 1), more while the GPU is not filled with this system's
-// atoms, but no more than its rows can keep busy (at least 8 row entries
-// per lane).
+// faster than 1), more while the system's lanes fit one resident wave of the
+// pair kernel (512 per SM; half of that beside an FP64 PME chain, whose
+// kernels run on the same SMs), but no more than its rows can keep busy (at
+// least 8 row entries per lane).  Steps of 8,788 LJ atoms (FP64) by lanes
+// 4 / 8 / 16 / 32: 30.0 / 28.0 / 30.8 / 34.2 us, of 55,296 55 / 60 / 69 / 90,
+// of 10,648 ions with PME 94 / 110 / 112 / 119.
 int Engine::lanes_for(const Slot& sl) const {
     if (lanes_fixed_ > 0)
         return lanes_fixed_;
     const long long n = sl.hp.n;
-    const long long target = (long long)num_sms_ * 2048 * 2;
+    const long long wave = (long long)num_sms_ * (sl.hp.has_pme && sl.hp.prec == kFP64 ? 256 : 512);
     int G = 4;
-    while (G < 32 && n * G < target)
+    while (G < 32 && n * G * 2 <= wave)
         G *= 2;
     int gmax = 1;
     while (gmax < 32 && gmax * 8 <= sl.mean_row)
