@@ -214,6 +214,8 @@ class Engine {
     LaunchCfg restricted_cfg(int id);
     void enqueue_step(bool profile, bool first, bool last);
     bool merge_halves() const;
+    bool fuse_scalars() const;
+    long long total_atoms() const;
     cudaGraphExec_t capture_steps(int steps);
     void widen_rows();
     int deform_budget(int n);

@@ -133,17 +133,16 @@ int fft_reg_cols(bool mixed);
 void launch_fft_reg(int pass, int idx, bool mixed, const ItemList& il, const SysParams* sp,
                     cudaStream_t s, bool pdl);
 // integrate.cu
-// fuse: the scalar updates of k_sys_a / k_sys_b run in the last block of each
-// system instead of a launch of their own.  cond_sort / cond_rows / use_cond:
-// the step graph's conditional handles of the list build (set when a system
-// rebuilds), only while the step is being captured
-void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse = false, bool pdl = false,
-                        cudaGraphConditionalHandle cond_sort = 0,
-                        cudaGraphConditionalHandle cond_rows = 0, bool use_cond = false);
-void launch_sys_a(const LaunchCfg& lc, cudaStream_t s);
+// fuse: the scalar updates run in the last block of each system's pass;
+// otherwise launch_sys follows (b: end of step, a: initial half; cond_sort /
+// cond_rows / use_cond: the step graph's conditional handles of the list
+// build, set when a system rebuilds)
+void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse = false, bool pdl = false);
 void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s, bool fuse = false, bool pdl = false);
-void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool pdl);
-void launch_sys_b(const LaunchCfg& lc, cudaStream_t s);
+void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl);
+void launch_sys(const LaunchCfg& lc, cudaStream_t s, bool b, bool a,
+                cudaGraphConditionalHandle cond_sort = 0,
+                cudaGraphConditionalHandle cond_rows = 0, bool use_cond = false);
 void launch_baro(const LaunchCfg& lc, cudaStream_t s);
 void launch_sys_energy(const LaunchCfg& lc, cudaStream_t s);
 void launch_force_rebuild(const LaunchCfg& lc, cudaStream_t s);

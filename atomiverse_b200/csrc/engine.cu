@@ -1268,7 +1268,7 @@ void Engine::enqueue_step_components() {
     };
     phase(ATVB_PHASE_INITIAL_INTEGRATE, [&] {
         launch_integrate_a(lc_, stream_);
-        launch_sys_a(lc_, stream_);
+        launch_sys(lc_, stream_, false, true);
     });
     phase(ATVB_PHASE_POST_INTEGRATE, [] {});
     phase(ATVB_PHASE_PRE_EXCHANGE, [] {});
@@ -1282,7 +1282,7 @@ void Engine::enqueue_step_components() {
     phase(ATVB_PHASE_POST_FORCE, [] {});
     phase(ATVB_PHASE_FINAL_INTEGRATE, [&] { launch_integrate_b(lc_, stream_); });
     phase(ATVB_PHASE_END_OF_STEP, [&] {
-        launch_sys_b(lc_, stream_);
+        launch_sys(lc_, stream_, true, false);
         launch_baro(lc_, stream_);
         if (lc_.any_snap)
             launch_snapshots(lc_, stream_);
@@ -1299,7 +1299,7 @@ int64_t Engine::rebuild_kernels() const {
 
 int64_t Engine::kernels_per_step() const {
     int64_t k = 0;
-    k += 1;                                   // integrate_a (with the scalar updates)
+    k += 1;                                   // integrate_a
     k += rebuild_kernels();                   // list build (rebuild steps only)
     for (int p = 0; p < 2; ++p)                // pair: one per lane class used
         for (int c = 0; c < kLaneClasses; ++c)
@@ -1308,8 +1308,9 @@ int64_t Engine::kernels_per_step() const {
     k += (lc_.pair_gen[0].n ? 1 : 0) + (lc_.pair_gen[1].n ? 1 : 0); // general pair
     if (!pme_slots_.empty())
         k += 2 + lc_.fft.launches();          // spread, gather, the transform passes
-    k += 1;                                   // integrate_b (with the scalar updates)
-    k += comps_.empty() ? 0 : 2;              // the scalar updates as their own kernels
+    k += 1;                                   // integrate_b
+    // the scalar updates as their own kernels
+    k += comps_.empty() && fuse_scalars() ? 0 : 2;
     k += lc_.any_snap ? 3 : 0;                // trajectory snapshots
     k += lc_.any_baro ? 1 : 0;                // Berendsen position scaling
     return k;
@@ -1398,17 +1399,25 @@ void Engine::capture_if(cudaGraphConditionalHandle h, F&& body) {
 void Engine::enqueue_step(bool profile, bool first, bool last) {
     const bool pdl = lc_.pdl, merge = !profile && merge_halves();
     const bool after_b = pdl && !first && !lc_.any_baro && !lc_.any_snap;
-    if (capturing_) {
+    // the conditional handles of a step are made before the kernel that sets
+    // them: k_integrate_a, or k_integrate_ba of the step before
+    auto new_handles = [&] {
         cudaStreamCaptureStatus st;
         unsigned long long id = 0;
         cudaGraph_t g = nullptr;
         CK(cudaStreamGetCaptureInfo(stream_, &st, &id, &g, nullptr, nullptr));
         CK(cudaGraphConditionalHandleCreate(&cond_sort_, g, 0, cudaGraphCondAssignDefault));
         CK(cudaGraphConditionalHandleCreate(&cond_rows_, g, 0, cudaGraphCondAssignDefault));
-    }
+    };
+    if (capturing_ && (first || !merge))
+        new_handles();
     prof_mark(profile, "integrate_a");
-    if (first || !merge)
-        launch_integrate_a(lc_, stream_, true, after_b, cond_sort_, cond_rows_, capturing_);
+    const bool fuse = fuse_scalars();
+    if (first || !merge) {
+        launch_integrate_a(lc_, stream_, fuse, after_b);
+        if (!fuse)
+            launch_sys(lc_, stream_, false, true, cond_sort_, cond_rows_, capturing_);
+    }
     prof_mark(profile, "neighbor");
     if (capturing_)
         capture_if(cond_sort_, [&](cudaStream_t cs) {
@@ -1421,10 +1430,17 @@ void Engine::enqueue_step(bool profile, bool first, bool last) {
     enqueue_forces(lc_, pme_slots_, profile, true, true);
     prof_mark(profile, "integrate_b");
     const bool after_pair = pdl && pme_slots_.empty();
-    if (last || !merge)
-        launch_integrate_b(lc_, stream_, true, after_pair);
-    else
-        launch_integrate_ba(lc_, stream_, after_pair);
+    if (last || !merge) {
+        launch_integrate_b(lc_, stream_, fuse, after_pair);
+        if (!fuse)
+            launch_sys(lc_, stream_, true, false);
+    } else {
+        if (capturing_)
+            new_handles();
+        launch_integrate_ba(lc_, stream_, fuse, after_pair);
+        if (!fuse)
+            launch_sys(lc_, stream_, true, true, cond_sort_, cond_rows_, capturing_);
+    }
     launch_baro(lc_, stream_);
     if (lc_.any_snap) {
         prof_mark(profile, "snapshot");
@@ -1583,6 +1599,18 @@ void Engine::run_pieces(int n, double* step_ms, double* total_ms) {
     steps_since_check_ += done;
 }
 
+// Whether the scalar updates run in the last block of the atom passes (small
+// engines, where a launch costs more than tickets) or as kernels.
+bool Engine::fuse_scalars() const { return total_atoms() < kCondMinAtoms; }
+
+long long Engine::total_atoms() const {
+    long long atoms = 0;
+    for (const auto& up : slots_)
+        if (up)
+            atoms += up->hp.n;
+    return atoms;
+}
+
 // Whether a graph of several steps may run the final half of a step and the
 // initial half of the next in one kernel (k_integrate_ba).
 bool Engine::merge_halves() const {
@@ -1594,18 +1622,14 @@ bool Engine::merge_halves() const {
             P.deform_axis >= 0 || P.stop_on_nan || P.snap_ring || P.ext_f)
             return false;
     }
-    return !capturing_; // conditional build nodes: k_integrate_a sets them
+    return true;
 }
 
 // The step graph: `steps` steps, captured from stream_.
 cudaGraphExec_t Engine::capture_steps(int steps) {
-    long long atoms = 0;
-    for (const auto& up : slots_)
-        if (up)
-            atoms += up->hp.n;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-    capturing_ = atoms >= kCondMinAtoms;
+    capturing_ = total_atoms() >= kCondMinAtoms;
     // programmatic launches only where a kernel does not fill the GPU: the
     // waiting blocks of the PME chain's next kernel would hold slots that
     // the pair kernel beside it can use (262,144 ions 2 % slower with them)
@@ -1645,10 +1669,10 @@ void Engine::ensure_graph() {
         gexec_ = capture_steps(1);
 }
 
-// Steps per launch of the longer graph a small engine gets once its work
-// lists have stood for kManyAfter steps (a server whose requests come and go
-// recaptures too often to pay for it): its programmatic launches also reach
-// from one step into the next.
+// Steps per launch of the longer graph an engine gets once its work lists
+// have stood for kManyAfter steps (a server whose requests come and go
+// recaptures too often to pay for it): launches reach from one step into the
+// next there (k_integrate_ba, and programmatic launches in small engines).
 constexpr int kManySteps = 8, kManyAfter = 24;
 
 void Engine::run_steps(int n) {
@@ -1666,17 +1690,14 @@ void Engine::run_steps(int n) {
         collect_profile();
     } else {
         ensure_graph();
-        long long atoms = 0;
-        for (const auto& up : slots_)
-            if (up)
-                atoms += up->hp.n;
         int k = 0;
-        if (atoms < kCondMinAtoms && n >= kManySteps && graph_steps_ >= kManyAfter) {
+        if (n >= kManySteps && graph_steps_ >= kManyAfter) {
             if (!gexec_many_)
                 gexec_many_ = capture_steps(kManySteps);
             for (; k + kManySteps <= n; k += kManySteps) {
                 CK(cudaGraphLaunch(gexec_many_, stream_));
-                merged_ += merge_halves() ? kManySteps - 1 : 0;
+                // a pass less per step, and a scalar kernel where there are any
+                merged_ += merge_halves() ? (fuse_scalars() ? 1 : 2) * (kManySteps - 1) : 0;
             }
         }
         for (; k < n; ++k)

@@ -203,36 +203,42 @@ __device__ __noinline__ void sys_a_update(const SysParams& P, SysState* st,
     }
 }
 
-// One thread per system, for steps whose scalar updates run as kernels of
-// their own (user components between the phases).
-__global__ void k_sys_a(const int* sys_list, int nsys, const SysParams* sp) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsys)
-        return;
-    const SysParams& P = sp[sys_list[k]];
-    SysState* gst = P.st;
-    if (gst->halted) {
-        gst->rebuild = 0; // nothing of this system moves: no list build either
-        return;
-    }
-    SysState loc = *gst;
-    sys_a_update(P, &loc, 0, 0, 0);
-    *gst = loc;
-}
-
-// The scalar updates of a system by the block that finishes the last of its
-// atom items (counted in `ticket`): the state and the parameters are copied
-// to shared memory by all threads, the state updated there by one and copied
-// back -- a launch of its own for this one thread per system took 6 to 10 us
-// of a small system's step.
-// The ticket's acquire-release orders the item's writes (sums, status and
-// rebuild flags) before it, and the last block's reads after every ticket.
 struct ScalarShared {
     SysState st;
     SysParams P;
     int last;
 };
 
+// One update of a system's state by a block: the state and the parameters
+// are copied to shared memory by all threads, the state updated there by one
+// and copied back.
+template <typename F>
+ATVB_DEV void scalar_update(const SysParams& P, ScalarShared& sh, F&& update) {
+    constexpr int words = (int)(sizeof(SysState) / sizeof(unsigned));
+    constexpr int pwords = (int)(sizeof(SysParams) / sizeof(unsigned));
+    unsigned* g = reinterpret_cast<unsigned*>(P.st);
+    unsigned* l = reinterpret_cast<unsigned*>(&sh.st);
+    const unsigned* gp = reinterpret_cast<const unsigned*>(&P);
+    unsigned* lp = reinterpret_cast<unsigned*>(&sh.P);
+    for (int k = threadIdx.x; k < words; k += blockDim.x)
+        l[k] = __ldcg(g + k);
+    for (int k = threadIdx.x; k < pwords; k += blockDim.x)
+        lp[k] = gp[k];
+    __syncthreads();
+    // an update that may commit a cell writes SysParams itself
+    const bool cell = sh.P.thermostat == kNPT || sh.P.baro || sh.P.deform_axis >= 0;
+    if (threadIdx.x == 0)
+        update(cell ? P : sh.P, &sh.st);
+    __syncthreads();
+    for (int k = threadIdx.x; k < words; k += blockDim.x)
+        g[k] = l[k];
+}
+
+// The scalar updates of a system by the block that finishes the last of its
+// atom items (counted in `ticket`) -- a launch of its own for this one thread
+// per system took 6 to 10 us of a small system's step.  The ticket's
+// acquire-release orders the item's writes (sums, status and rebuild flags)
+// before it, and the last block's reads after every ticket.
 template <typename F>
 ATVB_DEV void last_item(const SysParams& P, unsigned* ticket, ScalarShared& sh, F&& update) {
     __syncthreads(); // every thread's writes of this item come before the ticket
@@ -247,24 +253,7 @@ ATVB_DEV void last_item(const SysParams& P, unsigned* ticket, ScalarShared& sh, 
     }
     __syncthreads();
     if (sh.last) {
-        constexpr int words = (int)(sizeof(SysState) / sizeof(unsigned));
-        constexpr int pwords = (int)(sizeof(SysParams) / sizeof(unsigned));
-        unsigned* g = reinterpret_cast<unsigned*>(P.st);
-        unsigned* l = reinterpret_cast<unsigned*>(&sh.st);
-        const unsigned* gp = reinterpret_cast<const unsigned*>(&P);
-        unsigned* lp = reinterpret_cast<unsigned*>(&sh.P);
-        for (int k = threadIdx.x; k < words; k += blockDim.x)
-            l[k] = __ldcg(g + k);
-        for (int k = threadIdx.x; k < pwords; k += blockDim.x)
-            lp[k] = gp[k];
-        __syncthreads();
-        // an update that may commit a cell writes SysParams itself
-        const bool cell = sh.P.thermostat == kNPT || sh.P.baro || sh.P.deform_axis >= 0;
-        if (threadIdx.x == 0)
-            update(cell ? P : sh.P, &sh.st);
-        __syncthreads();
-        for (int k = threadIdx.x; k < words; k += blockDim.x)
-            g[k] = l[k];
+        scalar_update(P, sh, update);
         if (threadIdx.x == 0)
             *ticket = 0u;
     }
@@ -274,9 +263,7 @@ ATVB_DEV void last_item(const SysParams& P, unsigned* ticket, ScalarShared& sh, 
 // displacement check, KE of the kicked velocities (for Nose-Hoover); with
 // `fuse`, the last item of a system also runs its scalar updates.
 __global__ void __launch_bounds__(kChunk, 3)
-    k_integrate_a(const Item* items, int nitems, const SysParams* sp, int fuse,
-                  cudaGraphConditionalHandle cond_sort, cudaGraphConditionalHandle cond_rows,
-                  int use_cond) {
+    k_integrate_a(const Item* items, int nitems, const SysParams* sp, int fuse) {
     __shared__ double sh[32];
     __shared__ ScalarShared ss;
     pdl_sync();
@@ -351,7 +338,7 @@ __global__ void __launch_bounds__(kChunk, 3)
         }
         if (fuse)
             last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
-                sys_a_update(Q, st, cond_sort, cond_rows, use_cond);
+                sys_a_update(Q, st, 0, 0, 0);
             });
     }
 }
@@ -578,18 +565,29 @@ __device__ __noinline__ void sys_b_update(const SysParams& P, SysState* st) {
     st->step += 1;
 }
 
-// One thread per system (see k_sys_a).
-__global__ void k_sys_b(const int* sys_list, int nsys, const SysParams* sp) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsys)
+// The scalar updates as a kernel of their own, a block per system: steps with
+// user components between the phases, and engines whose atom passes are many
+// items long (the tickets and barriers of last_item cost 1,000,188 atoms 12
+// and 7 us a pass, this launch about 4).  B: end of step, A: initial half.
+constexpr int kSysThreads = 128;
+
+template <bool B, bool A>
+__global__ void __launch_bounds__(kSysThreads)
+    k_sys(const int* sys_list, const SysParams* sp, cudaGraphConditionalHandle cond_sort,
+          cudaGraphConditionalHandle cond_rows, int use_cond) {
+    __shared__ ScalarShared ss;
+    const SysParams& P = sp[sys_list[blockIdx.x]];
+    if (P.st->halted) {
+        if (A && threadIdx.x == 0)
+            P.st->rebuild = 0; // nothing of this system moves: no list build either
         return;
-    const SysParams& P = sp[sys_list[k]];
-    SysState* gst = P.st;
-    if (gst->halted)
-        return;
-    SysState loc = *gst;
-    sys_b_update(P, &loc);
-    *gst = loc;
+    }
+    scalar_update(P, ss, [&](const SysParams& Q, SysState* st) {
+        if (B)
+            sys_b_update(Q, st);
+        if (A)
+            sys_a_update(Q, st, cond_sort, cond_rows, use_cond);
+    });
 }
 
 // Langevin friction and random force of atom i at velocity v, added to f.
@@ -688,7 +686,7 @@ __global__ void __launch_bounds__(kChunk, 4)
 // bits, without writing and reading the velocities and forces in between
 // (204 bytes per atom instead of 296) and with one launch less per step.
 __global__ void __launch_bounds__(kChunk, 3)
-    k_integrate_ba(const Item* items, int nitems, const SysParams* sp) {
+    k_integrate_ba(const Item* items, int nitems, const SysParams* sp, int fuse) {
     __shared__ double sh[32];
     __shared__ ScalarShared ss;
     pdl_sync();
@@ -762,10 +760,11 @@ __global__ void __launch_bounds__(kChunk, 3)
         const double t = block_sum(ke, sh);
         if (threadIdx.x == 0)
             fix_add(&P.st->acc[kAccKEB], 0.5 * kMvv2e * t);
-        last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
-            sys_b_update(Q, st);
-            sys_a_update(Q, st, 0, 0, 0);
-        });
+        if (fuse)
+            last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
+                sys_b_update(Q, st);
+                sys_a_update(Q, st, 0, 0, 0);
+            });
     }
 }
 
@@ -1078,24 +1077,24 @@ void launch_npt_prep(const LaunchCfg& lc, cudaStream_t s) {
     k_npt_prep<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
 }
 
-void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl,
-                        cudaGraphConditionalHandle cond_sort,
-                        cudaGraphConditionalHandle cond_rows, bool use_cond) {
+void launch_integrate_a(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl) {
     launch_k(k_integrate_a, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp,
-             fuse ? 1 : 0, cond_sort, cond_rows, use_cond ? 1 : 0);
-}
-void launch_sys_a(const LaunchCfg& lc, cudaStream_t s) {
-    k_sys_a<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
+             fuse ? 1 : 0);
 }
 void launch_integrate_b(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl) {
     launch_k(k_integrate_b, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp,
              fuse ? 1 : 0);
 }
-void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
-    launch_k(k_integrate_ba, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp);
+void launch_integrate_ba(const LaunchCfg& lc, cudaStream_t s, bool fuse, bool pdl) {
+    launch_k(k_integrate_ba, lc.atoms.grid, kChunk, 0, s, pdl, lc.atoms.d, lc.atoms.n, lc.sp,
+             fuse ? 1 : 0);
 }
-void launch_sys_b(const LaunchCfg& lc, cudaStream_t s) {
-    k_sys_b<<<sys_blocks(lc.nsys), 128, 0, s>>>(lc.sys_list, lc.nsys, lc.sp);
+void launch_sys(const LaunchCfg& lc, cudaStream_t s, bool b, bool a,
+                cudaGraphConditionalHandle cond_sort, cudaGraphConditionalHandle cond_rows,
+                bool use_cond) {
+    const auto kernel = b && a ? k_sys<true, true> : b ? k_sys<true, false> : k_sys<false, true>;
+    kernel<<<lc.nsys, kSysThreads, 0, s>>>(lc.sys_list, lc.sp, cond_sort, cond_rows,
+                                           use_cond ? 1 : 0);
 }
 void launch_baro(const LaunchCfg& lc, cudaStream_t s) {
     if (lc.any_baro)
