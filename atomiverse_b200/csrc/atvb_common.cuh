@@ -58,6 +58,11 @@ enum Acc : int {
     kAccCount = 15
 };
 
+// The low words of the pair kernels' sums (SysParams::acc_lo), in units of
+// 2^-31 of the accumulators': LJ, Coulomb, six virials.
+constexpr int kAccLo = 8;
+constexpr double kAccLoScale = 2147483648.0; // 2^31
+
 struct SysState {
     unsigned long long acc[kAccCount]; // fixed-point accumulators
     double xi;         // Nose-Hoover friction
@@ -252,6 +257,7 @@ struct SysParams {
     // finished items of k_integrate_a / k_integrate_b: the block that
     // completes the last one runs the system's scalar updates
     unsigned* tickets;
+    unsigned long long* acc_lo; // kAccLo low words of the pair sums
     int *nbr, *nnbr;
     // PME buffers
     unsigned long long* grid_fix;

@@ -71,6 +71,7 @@ struct LaunchCfg {
     ItemList pme_real;  // kGridChunk real grid points per item
     const int* sys_list = nullptr; // device list of system indices
     int nsys = 0;
+    int pair_sums = 2;  // energy sums of the pair kernels (kAccLo with a virial)
     int pair_G = 4;     // lanes per atom of the largest system (reported)
     int any_mixed = 0, any_fp64 = 0;
     int any_snap = 0;   // a system publishes trajectory snapshots
@@ -100,6 +101,10 @@ inline void launch_k(void (*kernel)(KArgs...), int grid, int block, size_t smem,
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
     cuda_check(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...), "kernel launch");
+}
+
+inline size_t pair_smem(const LaunchCfg& lc) {
+    return (size_t)lc.pair_sums * 2 * kPairBlock * sizeof(long long);
 }
 
 // neighbor.cu

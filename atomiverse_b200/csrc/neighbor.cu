@@ -221,8 +221,7 @@ __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
 // five on every step of an engine too small for the conditional build nodes
 // (about 1 us each on the steps without a build), and on the steps with one
 // 14 us for 1,728 atoms and 23 for 4,000.  Up to 8,192 atoms: at 14,000 the
-// block took 68 us,
-// the five kernels 25.
+// block took 68 us, the five kernels 25.
 constexpr int kSortThreads = 1024, kSortBatch = 4;
 
 size_t small_sort_smem(int n, int ncell) {

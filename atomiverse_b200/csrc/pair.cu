@@ -143,16 +143,17 @@ ATVB_DEV void pair_term(const RowConst<T>& c, T dx, T dy, T dz, T qj,
 // Row of sorted atom s, lanes g, g+G, ...: two entries per iteration so that
 // both index loads and both position gathers are in flight together.
 template <bool LJ, bool CO, bool VIR, bool SHORT>
-ATVB_DEV void row_fp64(const SysParams& P, int s, int g, int G, PairAcc& acc) {
-    const double4* __restrict__ pos = reinterpret_cast<const double4*>(P.pos4);
+ATVB_DEV void row_fp64(const PairSys<double>& S, int s, int g, int G, PairAcc& acc) {
+    const double4* __restrict__ pos = S.pos;
     const double4 pi = pos[s];
-    const int nn = P.nnbr[s];
-    const int* __restrict__ row = P.nbr + (size_t)s * P.cap;
-    const RowConst<double> c = row_const<double>(P, pi.w);
+    const int nn = S.nnbr[s];
+    const int* __restrict__ row = S.nbr + (size_t)s * S.cap;
+    RowConst<double> c = S.c;
+    c.kqi = kQqr2e * pi.w;
     RowSums<double> a;
     bool near;
     // the wrapped 64-bit difference is the exact minimum-image separation
-    const double s0 = P.Lfix64[0], s1 = P.Lfix64[1], s2 = P.Lfix64[2];
+    const double s0 = S.step[0], s1 = S.step[1], s2 = S.step[2];
     auto sep = [&](const double4& pj, double& dx, double& dy, double& dz) {
         dx = (double)(__double_as_longlong(pi.x) - __double_as_longlong(pj.x)) * s0;
         dy = (double)(__double_as_longlong(pi.y) - __double_as_longlong(pj.y)) * s1;
@@ -229,13 +230,15 @@ ATVB_DEV void queue_near(const SysParams& P, int s, int code) {
 }
 
 template <bool LJ, bool CO, bool VIR, bool NEAR>
-ATVB_DEV void row_mixed(const SysParams& P, int s, int g, int G, PairAcc& acc) {
-    const int4* __restrict__ pos = reinterpret_cast<const int4*>(P.pos4);
+ATVB_DEV void row_mixed(const SysParams& P, const PairSys<float>& S, int s, int g, int G,
+                        PairAcc& acc) {
+    const int4* __restrict__ pos = S.pos;
     const int4 pi = pos[s];
-    const int nn = P.nnbr[s];
-    const int* __restrict__ row = P.nbr + (size_t)s * P.cap;
-    const float sx = P.Lf_fix[0], sy = P.Lf_fix[1], sz = P.Lf_fix[2];
-    const RowConst<float> c = row_const<float>(P, (double)__int_as_float(pi.w));
+    const int nn = S.nnbr[s];
+    const int* __restrict__ row = S.nbr + (size_t)s * S.cap;
+    const float sx = S.step[0], sy = S.step[1], sz = S.step[2];
+    RowConst<float> c = S.c;
+    c.kqi = (float)(kQqr2e * (double)__int_as_float(pi.w));
     RowSums<float> a;
     // the wrapped integer difference is the exact minimum-image separation
     auto sep = [&](const int4& pj, float& dx, float& dy, float& dz) {
@@ -279,58 +282,68 @@ ATVB_DEV void row_mixed(const SysParams& P, int s, int g, int G, PairAcc& acc) {
     finish_row(a, acc, VIR);
 }
 
-template <bool MIXED, bool LJ, bool CO, bool VIR>
-ATVB_DEV void row(const SysParams& P, int s, int g, int G, PairAcc& a) {
-    if (MIXED) {
-        // near-cutoff settling only where the LJ force jump matters
-        if (LJ && P.mix_band_lj > 0.0)
-            row_mixed<LJ, CO, VIR, true>(P, s, g, G, a);
-        else
-            row_mixed<LJ, CO, VIR, false>(P, s, g, G, a);
-    } else if (CO && P.coul_short) {
-        row_fp64<LJ, CO, VIR, true>(P, s, g, G, a);
-    } else {
-        row_fp64<LJ, CO, VIR, false>(P, s, g, G, a);
-    }
+template <bool LJ, bool CO, bool VIR>
+ATVB_DEV void row(const SysParams& P, const PairSys<float>& S, int s, int g, int G, PairAcc& a) {
+    // near-cutoff settling only where the LJ force jump matters
+    if (LJ && S.c.band_lj > 0.0f)
+        row_mixed<LJ, CO, VIR, true>(P, S, s, g, G, a);
+    else
+        row_mixed<LJ, CO, VIR, false>(P, S, s, g, G, a);
+}
+
+template <bool LJ, bool CO, bool VIR>
+ATVB_DEV void row(const SysParams& P, const PairSys<double>& S, int s, int g, int G, PairAcc& a) {
+    if (CO && P.coul_short)
+        row_fp64<LJ, CO, VIR, true>(S, s, g, G, a);
+    else
+        row_fp64<LJ, CO, VIR, false>(S, s, g, G, a);
 }
 
 template <bool MIXED, int G>
-__global__ void __launch_bounds__(256, MIXED ? 3 : 2)
-    k_pair(const Item* items, int nitems, const SysParams* sp) {
-    __shared__ double sh[32 * 8];
+__global__ void __launch_bounds__(kPairBlock, MIXED ? 3 : 2)
+    k_pair(const Item* items, int nitems, const SysParams* sp, int sums) {
+    using T = typename std::conditional<MIXED, float, double>::type;
+    extern __shared__ long long en_raw[];
+    const EnergyCols en = {en_raw, sums};
     pdl_sync();
     const int g = threadIdx.x % G;
     const int a_off = threadIdx.x / G;
-    PairAcc acc;
-    acc.elj = acc.ec = 0.0;
-    for (int k = 0; k < 6; ++k)
-        acc.v[k] = 0.0;
+    int cur = -1;
+    PairSys<T> S;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
-        if (P.prec != (MIXED ? kMixed : kFP64))
-            continue;
+        const bool first = item.sys != cur; // block-uniform
+        if (first) {
+            if (cur >= 0)
+                energy_flush(en, sp[cur], true);
+            cur = item.sys;
+            S = pair_sys<T>(P);
+        }
         const int s = item.begin + a_off;
-        acc.fx = acc.fy = acc.fz = 0.0;
-        if (s < P.n) {
-            const bool lj = P.has_lj, co = P.has_coul, vr = P.need_virial;
-            if (lj && co) {
-                if (vr)
-                    row<MIXED, true, true, true>(P, s, g, G, acc);
+        PairAcc acc;
+        acc.fx = acc.fy = acc.fz = acc.elj = acc.ec = 0.0;
+        for (int k = 0; k < 6; ++k)
+            acc.v[k] = 0.0;
+        if (s < S.n) {
+            if (S.lj && S.co) {
+                if (S.vir)
+                    row<true, true, true>(P, S, s, g, G, acc);
                 else
-                    row<MIXED, true, true, false>(P, s, g, G, acc);
-            } else if (lj) {
-                if (vr)
-                    row<MIXED, true, false, true>(P, s, g, G, acc);
+                    row<true, true, false>(P, S, s, g, G, acc);
+            } else if (S.lj) {
+                if (S.vir)
+                    row<true, false, true>(P, S, s, g, G, acc);
                 else
-                    row<MIXED, true, false, false>(P, s, g, G, acc);
-            } else if (co) {
-                if (vr)
-                    row<MIXED, false, true, true>(P, s, g, G, acc);
+                    row<true, false, false>(P, S, s, g, G, acc);
+            } else if (S.co) {
+                if (S.vir)
+                    row<false, true, true>(P, S, s, g, G, acc);
                 else
-                    row<MIXED, false, true, false>(P, s, g, G, acc);
+                    row<false, true, false>(P, S, s, g, G, acc);
             }
         }
+        energy_add(en, acc, S.vir, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) {
@@ -338,10 +351,11 @@ __global__ void __launch_bounds__(256, MIXED ? 3 : 2)
             fy += __shfl_xor_sync(0xffffffffu, fy, o);
             fz += __shfl_xor_sync(0xffffffffu, fz, o);
         }
-        if (g == 0 && s < P.n)
-            P.f4[s] = make_double4(fx, fy, fz, 0.0);
-        flush_energy(P, acc, sh);
+        if (g == 0 && s < S.n)
+            S.f4[s] = make_double4(fx, fy, fz, 0.0);
     }
+    if (cur >= 0)
+        energy_flush(en, sp[cur], false);
 }
 
 // Settles the near-cutoff pairs of the queued lane shares (one warp per
@@ -426,7 +440,8 @@ template <bool MIXED, int C>
 static void launch_pair_class(const LaunchCfg& lc, cudaStream_t s, bool& pdl) {
     const ItemList& L = lc.pair[MIXED ? 1 : 0][C];
     if (L.n) {
-        launch_k(k_pair<MIXED, 1 << C>, L.grid, kPairBlock, 0, s, pdl, L.d, L.n, lc.sp);
+        launch_k(k_pair<MIXED, 1 << C>, L.grid, kPairBlock, pair_smem(lc), s, pdl, L.d, L.n,
+                 lc.sp, lc.pair_sums);
         pdl = lc.pdl;
     }
     if constexpr (C + 1 < kLaneClasses)

@@ -166,25 +166,31 @@ ATVB_DEV void row_general(const SysParams& P, int s, int g, PairAcc& acc) {
 }
 
 template <bool MIXED>
-__global__ void __launch_bounds__(256)
-    k_pair_general(const Item* items, int nitems, const SysParams* sp) {
-    __shared__ double sh[32 * 8];
+__global__ void __launch_bounds__(kPairBlock)
+    k_pair_general(const Item* items, int nitems, const SysParams* sp, int sums) {
+    extern __shared__ long long en_raw[];
+    const EnergyCols en = {en_raw, sums};
     pdl_sync();
     const int g = threadIdx.x % kGenLanes;
     const int a_off = threadIdx.x / kGenLanes;
-    PairAcc acc;
-    acc.elj = acc.ec = 0.0;
-    for (int k = 0; k < 6; ++k)
-        acc.v[k] = 0.0;
+    int cur = -1;
     for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
         const Item item = items[it];
         const SysParams& P = sp[item.sys];
-        if (P.prec != (MIXED ? kMixed : kFP64))
-            continue;
+        const bool first = item.sys != cur; // block-uniform
+        if (first) {
+            if (cur >= 0)
+                energy_flush(en, sp[cur], true);
+            cur = item.sys;
+        }
         const int s = item.begin + a_off;
-        acc.fx = acc.fy = acc.fz = 0.0;
+        PairAcc acc;
+        acc.fx = acc.fy = acc.fz = acc.elj = acc.ec = 0.0;
+        for (int k = 0; k < 6; ++k)
+            acc.v[k] = 0.0;
         if (s < P.n)
             row_general<MIXED>(P, s, g, acc);
+        energy_add(en, acc, P.need_virial, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = kGenLanes / 2; o > 0; o >>= 1) {
@@ -194,18 +200,21 @@ __global__ void __launch_bounds__(256)
         }
         if (g == 0 && s < P.n)
             P.f4[s] = make_double4(fx, fy, fz, 0.0);
-        flush_energy(P, acc, sh);
     }
+    if (cur >= 0)
+        energy_flush(en, sp[cur], false);
 }
 
 void launch_pair_general(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
     const ItemList *D = &lc.pair_gen[0], *M = &lc.pair_gen[1];
     if (D->n) {
-        launch_k(k_pair_general<false>, D->grid, 256, 0, s, pdl, D->d, D->n, lc.sp);
+        launch_k(k_pair_general<false>, D->grid, kPairBlock, pair_smem(lc), s, pdl, D->d, D->n,
+                 lc.sp, lc.pair_sums);
         pdl = lc.pdl;
     }
     if (M->n)
-        launch_k(k_pair_general<true>, M->grid, 256, 0, s, pdl, M->d, M->n, lc.sp);
+        launch_k(k_pair_general<true>, M->grid, kPairBlock, pair_smem(lc), s, pdl, M->d, M->n,
+                 lc.sp, lc.pair_sums);
 }
 
 } // namespace atvb

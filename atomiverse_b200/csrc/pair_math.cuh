@@ -164,12 +164,27 @@ ATVB_DEV void finish_row(const RowSums<T>& r, PairAcc& a, bool vir) {
         a.fy = (double)r.fy;
         a.fz = (double)r.fz;
     }
-    a.elj += (double)r.elj;
-    a.ec += (double)r.ec;
+    a.elj = (double)r.elj;
+    a.ec = (double)r.ec;
     if (vir)
         for (int k = 0; k < 6; ++k)
-            a.v[k] += (double)r.v[k];
+            a.v[k] = (double)r.v[k];
 }
+
+// What a block reads of a system, once per system it works on (a row of 78
+// entries shared by four lanes spent a quarter of its loads on SysParams).
+template <typename T>
+struct PairSys {
+    using Pos = typename std::conditional<sizeof(T) == 4, int4, double4>::type;
+    const Pos* pos;
+    const int* nbr;
+    const int* nnbr;
+    double4* f4;
+    int n, cap;
+    bool lj, co, vir;
+    T step[3]; // length of one fixed-point position step per axis
+    RowConst<T> c;
+};
 
 template <typename T>
 ATVB_DEV RowConst<T> row_const(const SysParams& P, double qi) {
@@ -192,35 +207,85 @@ ATVB_DEV RowConst<T> row_const(const SysParams& P, double qi) {
     return c;
 }
 
-// Per-item flush: every item's energy/virial partial is rounded to fixed
-// point on its own, so a system's sums do not depend on which other systems
-// share the launch (results are identical alone and batched).
-ATVB_DEV void flush_energy(const SysParams& P, PairAcc& a, double* sh) {
-    if (P.need_virial) {
-        double v[8] = {a.elj, a.ec, a.v[0], a.v[1], a.v[2], a.v[3], a.v[4], a.v[5]};
-        block_sum_vec<8>(v, sh);
-        if (threadIdx.x == 0) {
-            if (P.has_lj)
-                fix_add(&P.st->acc[kAccELJ], 0.5 * v[0]);
-            if (P.has_coul)
-                fix_add(&P.st->acc[kAccECoul], 0.5 * v[1]);
-            for (int k = 0; k < 6; ++k)
-                fix_add(&P.st->acc[kAccVir + k], 0.5 * v[2 + k]);
+template <typename T>
+ATVB_DEV PairSys<T> pair_sys(const SysParams& P) {
+    PairSys<T> S;
+    S.pos = reinterpret_cast<const typename PairSys<T>::Pos*>(P.pos4);
+    S.nbr = P.nbr;
+    S.nnbr = P.nnbr;
+    S.f4 = P.f4;
+    S.n = P.n;
+    S.cap = P.cap;
+    S.lj = P.has_lj;
+    S.co = P.has_coul;
+    S.vir = P.need_virial;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        S.step[d] = sizeof(T) == 4 ? (T)P.Lf_fix[d] : (T)P.Lfix64[d];
+    S.c = row_const<T>(P, 0.0);
+    return S;
+}
+
+// Energies and virials of a block: each lane rounds its share of a row to
+// fixed point on its own, in two words (2^-32 eV, and the rest in 2^-63 eV),
+// and adds them to its own columns of shared memory, so a system's sums
+// depend neither on the order nor on which other systems share the launch;
+// the columns go to the system once per block and system.  (A block sum per
+// item cost two barriers and up to 80 shuffles per 64 atoms.)
+// The columns are dynamic shared memory, `sums` of them (2, or all kAccLo if
+// a system of the launch needs its virial): what they take is L1 the gathers
+// do not have.
+struct EnergyCols {
+    long long* v; // [sum][word][thread]
+    int sums;
+    ATVB_DEV long long& at(int k, int word) const {
+        return v[(2 * k + word) * kPairBlock + threadIdx.x];
+    }
+};
+
+// v into this lane's column of sum k: the first of a system stores.
+ATVB_DEV void energy_add1(const EnergyCols& e, int k, double v, bool first) {
+    const double t = v * (0.5 * kEFix); // 1/2: every pair is visited from both of its atoms
+    const long long h = __double2ll_rn(t);
+    const long long l = __double2ll_rn((t - (double)h) * kAccLoScale);
+    e.at(k, 0) = first ? h : e.at(k, 0) + h;
+    e.at(k, 1) = first ? l : e.at(k, 1) + l;
+}
+
+// The row share of every lane of the block (zeros past the last atom).
+ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool vir, bool first) {
+    energy_add1(e, 0, a.elj, first);
+    energy_add1(e, 1, a.ec, first);
+    if (vir && e.sums == kAccLo)
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            energy_add1(e, 2 + k, a.v[k], first);
+}
+
+// Block-uniform.  `again`: the block goes on to another system.
+ATVB_DEV void energy_flush(const EnergyCols& e, const SysParams& P, bool again) {
+    __syncthreads();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    static_assert(kPairBlock / 32 >= kAccLo, "a warp per sum");
+    if (w < (P.need_virial ? e.sums : 2)) {
+        long long h = 0, l = 0;
+#pragma unroll
+        for (int k = 0; k < kPairBlock / 32; ++k) {
+            h += e.v[2 * w * kPairBlock + k * 32 + lane];
+            l += e.v[(2 * w + 1) * kPairBlock + k * 32 + lane];
         }
-    } else {
-        double v[2] = {a.elj, a.ec};
-        block_sum_vec<2>(v, sh);
-        if (threadIdx.x == 0) {
-            // 1/2: every pair is visited from both of its atoms
-            if (P.has_lj)
-                fix_add(&P.st->acc[kAccELJ], 0.5 * v[0]);
-            if (P.has_coul)
-                fix_add(&P.st->acc[kAccECoul], 0.5 * v[1]);
+        h = warp_sum(h);
+        l = warp_sum(l);
+        const int acc = w == 0 ? kAccELJ : w == 1 ? kAccECoul : kAccVir + w - 2;
+        if (lane == 0) {
+            if (h)
+                red_add_u64(&P.st->acc[acc], (unsigned long long)h);
+            if (l)
+                red_add_u64(&P.acc_lo[w], (unsigned long long)l);
         }
     }
-    a.elj = a.ec = 0.0;
-    for (int k = 0; k < 6; ++k)
-        a.v[k] = 0.0;
+    if (again)
+        __syncthreads();
 }
 
 // Mixed: at least 3 resident blocks (80 registers); FP64: 2.
