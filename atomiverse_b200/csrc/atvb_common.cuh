@@ -253,7 +253,7 @@ struct SysParams {
     int *perm, *rank, *cell_of, *slot, *cell_count, *cell_start;
     int* cell_sums; // atoms per kScanChunk cells
     int2* perm0;    // {atom, fixed-point z} by cell, in arrival order (k_cell_scatter)
-    int small_sort; // the whole cell sort in one block (k_sort_small)
+    int small_sort; // the whole cell sort in one cluster (k_sort_small)
     // finished items of k_integrate_a / k_integrate_b: the block that
     // completes the last one runs the system's scalar updates
     unsigned* tickets;

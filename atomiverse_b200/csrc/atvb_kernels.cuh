@@ -13,8 +13,8 @@ constexpr long long kCondMinAtoms = 100000; // engines from this size skip them 
                                             // conditional graph nodes
 constexpr int kListChunk = 4;   // warp tasks per item of the list build
 constexpr int kScanChunk = 2048; // cells per item of the cell scan
-// largest system whose cell sort runs in one block (k_sort_small)
-constexpr int kSortSmallAtoms = 8192, kSortSmallCells = 16384;
+constexpr int kSortSmallAtoms = 65536; // largest system whose cell sort runs in one
+                                       // cluster (k_sort_small)
 constexpr int kGridChunk = 4096; // grid points per item of the PME grid kernels
 constexpr int kLaneClasses = 6;  // pair lanes per atom: 1, 2, 4, 8, 16, 32
 constexpr int kGenLanes = 8;      // lanes per atom of k_pair_general
@@ -57,11 +57,10 @@ struct LaunchCfg {
     ItemList pair[2][kLaneClasses];
     ItemList pair_gen[2]; // [precision]: systems with types or special pairs
                           // (kChunk / kGenLanes atoms per item)
-    // the cell sort: systems sorted by one block each (small_list, nsmall;
-    // small_smem bytes for the largest), and the items of the others
+    // the cell sort: systems sorted by one cluster each (small_list, nsmall),
+    // and the items of the others
     const int* small_list = nullptr;
     int nsmall = 0;
-    size_t small_smem = 0;
     ItemList sort_atoms; // kChunk atoms per item
     ItemList scan;       // kScanChunk cells per item
     // kernels of the chain launched as programmatic dependents (step graphs)
@@ -108,9 +107,6 @@ inline size_t pair_smem(const LaunchCfg& lc) {
 }
 
 // neighbor.cu
-bool small_sort_fits(int n, int ncell);
-size_t small_sort_smem(int n, int ncell);
-void sort_smem_optin();
 void launch_rebuild(const LaunchCfg& lc, cudaStream_t s);
 // `pdl` of a launcher: whether its first kernel depends on the launch before
 // it alone (the rest of its chain follows lc.pdl)

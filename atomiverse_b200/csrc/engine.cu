@@ -449,7 +449,6 @@ void Slot::replan_cells(double shrink) {
         hp.npt_Lmin[k] = geo.Lmin[k];
     }
     hp.ncell = geo.nc[0] * geo.nc[1] * geo.nc[2];
-    hp.small_sort = small_sort_fits(hp.n, hp.ncell) ? 1 : 0;
     hp.ncol = (int)geo.cols.size();
     hp.cell_count = (int*)dalloc(sizeof(int) * hp.ncell);
     hp.cell_start = (int*)dalloc(sizeof(int) * (hp.ncell + 1));
@@ -641,7 +640,7 @@ Slot::Slot(const atvb_system_desc& d, const DevMem& mem) : desc(d), mem_(mem) {
     hp.cell_of = di(n);
     hp.slot = di(n);
     hp.perm0 = (int2*)dalloc((size_t)n * sizeof(int2));
-    hp.small_sort = small_sort_fits(n, hp.ncell) ? 1 : 0;
+    hp.small_sort = n <= kSortSmallAtoms ? 1 : 0;
     hp.tickets = (unsigned*)dalloc(2 * sizeof(unsigned));
     CK(cudaMemsetAsync(hp.tickets, 0, 2 * sizeof(unsigned), stream));
     hp.acc_lo = (unsigned long long*)dalloc(kAccLo * sizeof(unsigned long long));
@@ -764,7 +763,6 @@ Engine::Engine(int device) : device_(device) {
     CK(cudaEventCreateWithFlags(&pme_join_, cudaEventDisableTiming));
     // the FFT blocks' line buffers live in dynamic shared memory above 48 KB
     fft_smem_optin(kFftSmem + 1024);
-    sort_smem_optin();
     stage_ = std::make_unique<HostStage>(device);
 }
 
@@ -998,7 +996,6 @@ void Engine::build_lists() {
     list_allocs_.clear();
     std::vector<Item> atoms, list, sort_atoms, scan, patoms;
     std::vector<int> sys, small;
-    size_t small_smem = 0;
     std::vector<Item> pair_by[2][kLaneClasses];
     std::vector<Item> pair_gen[2];
     lc_ = LaunchCfg{};
@@ -1039,7 +1036,6 @@ void Engine::build_lists() {
         }
         if (P.small_sort) {
             small.push_back(k);
-            small_smem = std::max(small_smem, small_sort_smem(P.n, P.ncell));
         } else {
             for (int b = 0; b < P.n; b += kChunk)
                 sort_atoms.push_back({k, b});
@@ -1082,7 +1078,6 @@ void Engine::build_lists() {
     lc_.sort_atoms = make_list(list_allocs_, sort_atoms, g_light, mem_);
     lc_.scan = make_list(list_allocs_, scan, g_light, mem_);
     lc_.nsmall = (int)small.size();
-    lc_.small_smem = small_smem;
     if (!small.empty()) {
         void* p = mem_.alloc(sizeof(int) * small.size());
         list_allocs_.push_back(p);
@@ -1914,7 +1909,6 @@ LaunchCfg Engine::restricted_cfg(int id) {
     c.nsys = 1;
     c.nsmall = P.small_sort ? 1 : 0;
     c.small_list = c.sys_list;
-    c.small_smem = small_sort_smem(P.n, P.ncell);
     single_[id] = {list_epoch_, c};
     return c;
 }

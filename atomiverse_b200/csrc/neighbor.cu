@@ -190,7 +190,7 @@ __global__ void k_cell_scatter(const Item* items, int nitems,
 ATVB_DEV int sorted_place(const int2* perm0, int a, int b, int2 me) {
     int s = a;
     for (int k = a; k < b; ++k) {
-        const int2 o = perm0[k];
+        const int2 o = __ldcg(perm0 + k);
         s += (unsigned)o.y < (unsigned)me.y || (o.y == me.y && o.x < me.x) ? 1 : 0;
     }
     return s;
@@ -216,55 +216,55 @@ __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
     }
 }
 
-// The whole cell sort of a small system (small_sort_fits) in one block, the
-// cell counts and the cells' atoms in shared memory: one launch instead of
-// five on every step of an engine too small for the conditional build nodes
-// (about 1 us each on the steps without a build), and on the steps with one
-// 14 us for 1,728 atoms and 23 for 4,000.  Up to 8,192 atoms: at 14,000 the
-// block took 68 us, the five kernels 25.
-constexpr int kSortThreads = 1024, kSortBatch = 4;
+// The whole cell sort of a system of at most kSortSmallAtoms atoms in one
+// cluster of eight blocks, with cluster barriers between the stages: one
+// launch instead of five on every step of an engine too small for the
+// conditional build nodes (about 1 us each on the steps without a build).
+// Per pass against one block up to 8,192 atoms and five kernels above: 4,000
+// atoms 2.48 -> 2.38 ms, 13,500 2.38 -> 2.20, 14,039 2.17 -> 2.00, 22,176
+// ions 4.64 -> 4.46; 256 atoms 1.91 -> 1.95 (the cluster's launch).
+// Data of other blocks of the cluster is read past L1 (__ldcg).
+constexpr int kSortThreads = 1024, kSortCtas = 8;
 
-size_t small_sort_smem(int n, int ncell) {
-    return (size_t)n * sizeof(int2) + ((size_t)ncell + 1) * sizeof(int);
+ATVB_DEV void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kSortThreads)
+// The int at `p` of this block's shared memory, in block `rank` of the cluster.
+ATVB_DEV int cluster_peek(const int* p, int rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(r) : "memory");
+    return v;
+}
+
+__global__ void __cluster_dims__(kSortCtas, 1, 1) __launch_bounds__(kSortThreads)
     k_sort_small(const int* sys_list, const SysParams* sp) {
-    extern __shared__ int2 keys[]; // n {atom, fixed-point z}, then ncell + 1 counts
     __shared__ int tot[kSortThreads / 32];
+    __shared__ int cta_total;
     pdl_sync();
-    const SysParams& P = sp[sys_list[blockIdx.x]];
+    const SysParams& P = sp[sys_list[blockIdx.x / kSortCtas]];
     if (!P.st->rebuild)
-        return;
+        return; // the whole cluster
+    constexpr int T = kSortCtas * kSortThreads;
     const int n = P.n, ncell = P.ncell, tid = threadIdx.x;
+    const int rank = blockIdx.x % kSortCtas, gtid = rank * kSortThreads + tid;
     const int lane = tid & 31, w = tid >> 5;
-    int* cnt = reinterpret_cast<int*>(keys + n);
-    for (int c = tid; c < ncell; c += kSortThreads)
-        cnt[c] = 0;
-    __syncthreads();
-    int* const cell_of = P.cell_of;
-    int* const slot = P.slot;
-    for (int i0 = tid; i0 < n; i0 += kSortBatch * kSortThreads) {
-        int c[kSortBatch]; // loads of a batch before its stores
-#pragma unroll
-        for (int k = 0; k < kSortBatch; ++k)
-            c[k] = i0 + k * kSortThreads < n ? cell_index(P, i0 + k * kSortThreads) : 0;
-#pragma unroll
-        for (int k = 0; k < kSortBatch; ++k) {
-            const int i = i0 + k * kSortThreads;
-            if (i < n) {
-                cell_of[i] = c[k];
-                slot[i] = atomicAdd(&cnt[c[k]], 1);
-            }
-        }
+    for (int i = gtid; i < n; i += T) {
+        const int c = cell_index(P, i);
+        P.cell_of[i] = c;
+        P.slot[i] = atomicAdd(&P.cell_count[c], 1);
     }
-    __syncthreads();
-    // exclusive scan: each thread a run of cells, then the runs' totals
-    const int per = (ncell + kSortThreads - 1) / kSortThreads;
-    const int c0 = min(tid * per, ncell), c1 = min(c0 + per, ncell);
+    cluster_barrier();
+    // exclusive scan: each thread a run of cells, the runs' totals within the
+    // block, the blocks' totals within the cluster
+    const int per = (ncell + T - 1) / T;
+    const int c0 = min(gtid * per, ncell), c1 = min(c0 + per, ncell);
     int sum = 0;
     for (int c = c0; c < c1; ++c)
-        sum += cnt[c];
+        sum += __ldcg(P.cell_count + c);
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -284,40 +284,32 @@ __global__ void __launch_bounds__(kSortThreads)
                 t += u;
         }
         tot[lane] = t;
+        if (lane == 31)
+            cta_total = t;
     }
-    __syncthreads();
+    cluster_barrier();
     int base = incl - sum + (w > 0 ? tot[w - 1] : 0);
+    for (int r = 0; r < rank; ++r)
+        base += cluster_peek(&cta_total, r);
     for (int c = c0; c < c1; ++c) {
-        const int v = cnt[c];
-        cnt[c] = base;
+        const int v = __ldcg(P.cell_count + c);
         P.cell_start[c] = base;
+        P.cell_count[c] = 0; // ready for the next rebuild
         base += v;
     }
-    if (tid == 0) {
-        cnt[ncell] = n;
+    if (gtid == 0)
         P.cell_start[ncell] = n;
-    }
-    __syncthreads();
-    const double fz = P.fix_scale[2];
-    const double* const z = P.z;
-#pragma unroll 4
-    for (int i = tid; i < n; i += kSortThreads)
-        keys[cnt[cell_of[i]] + slot[i]] = make_int2(i, (int)pos_fix(z[i], fz));
-    __syncthreads();
-    for (int i0 = tid; i0 < n; i0 += kSortBatch * kSortThreads) {
-        int s[kSortBatch];
-#pragma unroll
-        for (int k = 0; k < kSortBatch; ++k) {
-            const int i = i0 + k * kSortThreads;
-            if (i < n) {
-                const int c = cell_of[i];
-                s[k] = sorted_place(keys, cnt[c], cnt[c + 1], make_int2(i, (int)pos_fix(z[i], fz)));
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kSortBatch; ++k)
-            if (i0 + k * kSortThreads < n)
-                sorted_record(P, i0 + k * kSortThreads, s[k]);
+    cluster_barrier();
+    for (int i = gtid; i < n; i += T) // cell and slot of this thread's own atoms
+        P.perm0[__ldcg(P.cell_start + P.cell_of[i]) + P.slot[i]] =
+            make_int2(i, (int)pos_fix(P.z[i], P.fix_scale[2]));
+    cluster_barrier();
+    for (int t = gtid; t < n; t += T) {
+        const int2 me = __ldcg(P.perm0 + t);
+        const int c = __ldcg(P.cell_of + me.x);
+        sorted_record(P, me.x,
+                      sorted_place(P.perm0, __ldcg(P.cell_start + c), __ldcg(P.cell_start + c + 1),
+                                   me));
     }
 }
 
@@ -685,20 +677,12 @@ __global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
         flush();
 }
 
-bool small_sort_fits(int n, int ncell) { return n <= kSortSmallAtoms && ncell <= kSortSmallCells; }
-
-void sort_smem_optin() {
-    cuda_check(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)small_sort_smem(kSortSmallAtoms, kSortSmallCells)),
-               "shared memory of k_sort_small");
-}
-
 // Binning and the sorted repack: after these the sorted positions (pos4)
 // that the PME chain reads are final, so that chain may start beside the
 // list build.
 void launch_sort_cells(const LaunchCfg& lc, cudaStream_t s, bool pdl) {
     if (lc.nsmall) {
-        launch_k(k_sort_small, lc.nsmall, kSortThreads, lc.small_smem, s, pdl, lc.small_list,
+        launch_k(k_sort_small, lc.nsmall * kSortCtas, kSortThreads, 0, s, pdl, lc.small_list,
                  lc.sp);
         pdl = lc.pdl;
     }

@@ -387,7 +387,7 @@ int atvb_system_profile_read(atvb_system* sys, atvb_kernel_time* out,
 /* Lanes per atom in the pair kernel (1,2,4,8,16,32); 0 = autotune. */
 int atvb_system_set_pair_lanes(atvb_system* sys, int32_t lanes);
 /* Kernel launches of the last step() call, counting the list-build kernels on
- * every step (six; two if every system has at most 8,192 atoms, seven if
+ * every step (six; two if every system has at most 65,536 atoms, seven if
  * systems on both sides of that share an engine): in the step graph of a
  * system (or batch) of at least 100,000 atoms they launch only on steps
  * where a system rebuilds its list (conditional nodes), so the launches made
