@@ -88,7 +88,7 @@ struct SysState {
     double pressure;   // (2 KE + trace W) / (3 V) [eV/A^3]
     // MTK NPT extended state (nose_hoover_npt.cpp): chains, strain rates and
     // the factors of the next initial half step, prepared at the end of the
-    // previous step by k_sys_b (or by k_npt_prep before the first step)
+    // previous step by sys_b_update (or by k_npt_prep before the first step)
     double eta_t[kMaxChain], eta_t_dot[kMaxChain];
     double eta_b[kMaxChain], eta_b_dot[kMaxChain];
     double eps_dot[3];

@@ -1,6 +1,6 @@
 // box.cuh -- every SysParams field that depends on the cell edges, computed
 // in one place for the host (system setup) and the device (the MTK NPT cell
-// update, committed once per step by k_sys_a).
+// update, committed once per step by sys_a_update).
 //
 // Depends on the cell: the fixed-point position scales, the minimum-image
 // constants, the bin size (the bin COUNT is fixed when the system is

@@ -5,7 +5,7 @@
 // (src/cuda/driver/driver.cu:123-157), which walks ten phases and launches
 // every component kernel from the host each step.  Here a step is one CUDA
 // graph launch: the phase order is fixed at capture time and the neighbour
-// rebuild decision is taken on the device (k_sys_a), so the loop has no
+// rebuild decision is taken on the device (sys_a_update), so the loop has no
 // host synchronisation.  An Engine holds any number of systems; the
 // single-system API is an Engine with one slot, the batch API an Engine
 // with many, and the server an Engine whose slots come and go.
@@ -1389,7 +1389,7 @@ void Engine::capture_if(cudaGraphConditionalHandle h, F&& body) {
 
 // One step.  In the captured graph of an engine with at least
 // kCondMinAtoms atoms the list-build kernels sit in two IF nodes whose
-// handles k_sys_a sets when any system builds its list (reset at every
+// handles sys_a_update sets when any system builds its list (reset at every
 // launch): the cell sort before the PME branch forks, the list build beside
 // it; on other steps they do not launch.  Measured on the B200: 262,144
 // ions +0.8 %, 1,000,188 LJ atoms +7 %; but 4,000 and 10,648 atoms -13 %

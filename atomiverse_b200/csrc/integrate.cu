@@ -9,7 +9,7 @@
 //   (fix_langevin.cpp:79-155), final_integrate: v += dt/2 f/m; NH again;
 //   end_of_step: KE (init.cpp:29-45).
 // Fusion: the thermostat scale of each half is a per-system scalar produced
-// by a one-thread-per-system kernel; it is applied to v by the NEXT atom
+// by sys_a_update or sys_b_update; it is applied to v by the NEXT atom
 // pass (the initial-half scale by the final kick, the final-half scale by
 // the next step's initial kick), so each half step reads and writes v once.
 // The end-of-step kinetic energy is s_B^2 * KE(v) for the deferred scale.
@@ -473,7 +473,7 @@ ATVB_DEV void berendsen(const SysParams& P, SysState* st) {
 // the k-th deformation step takes the axis edge from L0 (1 + r dt (k-1)) to
 // L0 (1 + r dt k) (engineering strain, linear in time) and scales positions
 // along it by the same ratio.  Folded into the next initial half's drift
-// (x s + v dt s along the axis, in the new cell); k_sys_a commits the cell.
+// (x s + v dt s along the axis, in the new cell); sys_a_update commits the cell.
 ATVB_DEV void deform_prepare(const SysParams& P, SysState* st, long long k) {
     const int ax = P.deform_axis;
     const double rdt = P.deform_rate * P.dt;

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 3 : 2)
                     row<false, true, false>(P, S, s, g, G, acc);
             }
         }
-        energy_add(en, acc, S.vir, first);
+        energy_add(en, acc, S.lj, S.co, S.vir, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) {
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 3 : 2)
 // matter; energy and virial corrections go to the fixed-point accumulators
 // (x 1/2: each pair sits in both of its rows).  Runs after the pair kernel
 // and before the PME gather adds to the same forces.  The queue is emptied
-// at the start of the next step (k_sys_a) or force pass.
+// at the start of the next step (sys_a_update) or force pass.
 constexpr int kFixBlocks = 16;
 
 template <bool LJ, bool CO, bool VIR>

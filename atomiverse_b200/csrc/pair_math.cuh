@@ -253,9 +253,12 @@ ATVB_DEV void energy_add1(const EnergyCols& e, int k, double v, bool first) {
 }
 
 // The row share of every lane of the block (zeros past the last atom).
-ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool vir, bool first) {
-    energy_add1(e, 0, a.elj, first);
-    energy_add1(e, 1, a.ec, first);
+ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool lj, bool co, bool vir,
+                         bool first) {
+    if (lj)
+        energy_add1(e, 0, a.elj, first);
+    if (co)
+        energy_add1(e, 1, a.ec, first);
     if (vir && e.sums == kAccLo)
 #pragma unroll
         for (int k = 0; k < 6; ++k)
@@ -267,7 +270,7 @@ ATVB_DEV void energy_flush(const EnergyCols& e, const SysParams& P, bool again) 
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     static_assert(kPairBlock / 32 >= kAccLo, "a warp per sum");
-    if (w < (P.need_virial ? e.sums : 2)) {
+    if (w == 0 ? P.has_lj : w == 1 ? P.has_coul : P.need_virial && w < e.sums) {
         long long h = 0, l = 0;
 #pragma unroll
         for (int k = 0; k < kPairBlock / 32; ++k) {
