@@ -13,7 +13,8 @@
 // so the force on every atom is summed in the same order on every run (no
 // atomics on forces).  Because every pair appears in both rows, energy and
 // virial carry a factor 1/2 (pair_lj_cut.cu:195 in the reference does the
-// same on its full list).  Energy/virial block partials are added into the
+// same on its full list).  Energies and virials are summed per lane in two-word
+// fixed point and added once per block and system into the
 // system's 64-bit fixed-point accumulators.
 //
 // erfc: erfc(x) = exp(-x^2) erfcx(x), with erfcx from ONE polynomial in
@@ -237,8 +238,9 @@ ATVB_DEV void row_mixed(const SysParams& P, const PairSys<float>& S, int s, int 
     const int nn = S.nnbr[s];
     const int* __restrict__ row = S.nbr + (size_t)s * S.cap;
     const float sx = S.step[0], sy = S.step[1], sz = S.step[2];
-    RowConst<float> c = S.c;
-    c.kqi = (float)(kQqr2e * (double)__int_as_float(pi.w));
+    // constants from SysParams per row: kept live across rows they cost this
+    // kernel registers (262,144 ions 361 us a launch with PairSys's, 332 so)
+    const RowConst<float> c = row_const<float>(P, (double)__int_as_float(pi.w));
     RowSums<float> a;
     // the wrapped integer difference is the exact minimum-image separation
     auto sep = [&](const int4& pj, float& dx, float& dy, float& dz) {
@@ -285,7 +287,7 @@ ATVB_DEV void row_mixed(const SysParams& P, const PairSys<float>& S, int s, int 
 template <bool LJ, bool CO, bool VIR>
 ATVB_DEV void row(const SysParams& P, const PairSys<float>& S, int s, int g, int G, PairAcc& a) {
     // near-cutoff settling only where the LJ force jump matters
-    if (LJ && S.c.band_lj > 0.0f)
+    if (LJ && P.mix_band_lj > 0.0)
         row_mixed<LJ, CO, VIR, true>(P, S, s, g, G, a);
     else
         row_mixed<LJ, CO, VIR, false>(P, S, s, g, G, a);
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 3 : 2)
                     row<false, true, false>(P, S, s, g, G, acc);
             }
         }
-        energy_add(en, acc, S.lj, S.co, S.vir, first);
+        energy_add(en, acc, S.vir, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) {

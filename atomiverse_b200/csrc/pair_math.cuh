@@ -172,7 +172,8 @@ ATVB_DEV void finish_row(const RowSums<T>& r, PairAcc& a, bool vir) {
 }
 
 // What a block reads of a system, once per system it works on (a row of 78
-// entries shared by four lanes spent a quarter of its loads on SysParams).
+// entries shared by four lanes spent a quarter of its loads on SysParams);
+// the mixed rows use the pointers only.
 template <typename T>
 struct PairSys {
     using Pos = typename std::conditional<sizeof(T) == 4, int4, double4>::type;
@@ -253,12 +254,11 @@ ATVB_DEV void energy_add1(const EnergyCols& e, int k, double v, bool first) {
 }
 
 // The row share of every lane of the block (zeros past the last atom).
-ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool lj, bool co, bool vir,
-                         bool first) {
-    if (lj)
-        energy_add1(e, 0, a.elj, first);
-    if (co)
-        energy_add1(e, 1, a.ec, first);
+// The LJ and Coulomb sums unconditionally: skipping one the system has not
+// made the mixed kernel spill (347 -> 361 us at 262,144 ions).
+ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool vir, bool first) {
+    energy_add1(e, 0, a.elj, first);
+    energy_add1(e, 1, a.ec, first);
     if (vir && e.sums == kAccLo)
 #pragma unroll
         for (int k = 0; k < 6; ++k)
@@ -270,7 +270,7 @@ ATVB_DEV void energy_flush(const EnergyCols& e, const SysParams& P, bool again) 
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     static_assert(kPairBlock / 32 >= kAccLo, "a warp per sum");
-    if (w == 0 ? P.has_lj : w == 1 ? P.has_coul : P.need_virial && w < e.sums) {
+    if (w < (P.need_virial ? e.sums : 2)) {
         long long h = 0, l = 0;
 #pragma unroll
         for (int k = 0; k < kPairBlock / 32; ++k) {

@@ -10,7 +10,7 @@
 // device memory released.  Positions, velocities, neighbour lists and PME
 // grids stay resident on the device between ticks.  A system's arithmetic
 // does not depend on which other systems share the launch (per-atom work,
-// fixed-point sums flushed per work item), so a request's result is the same
+// fixed-point sums exact in any order), so a request's result is the same
 // alone and in the mix.
 #include <algorithm>
 #include <cstring>
