@@ -162,23 +162,26 @@ ATVB_DEV void row_fp64(const PairSys<double>& S, int s, int g, int G, PairAcc& a
     };
     // software pipeline: the positions of the next two entries and the row
     // indices of the two after them are in flight while the current pair
-    // computes (the kernel waits on the gather, not on the FP64 pipe)
+    // computes (the kernel waits on the gather, not on the FP64 pipe).  Rows
+    // are read by plain loads: as a programmatic dependent this grid is
+    // resident while k_build_list still writes them, which the read-only
+    // path (__ldg) does not allow
     int k = g;
-    int ja = k < nn ? __ldg(row + k) : 0;
-    int jb = k + G < nn ? __ldg(row + k + G) : 0;
+    int ja = k < nn ? row[k] : 0;
+    int jb = k + G < nn ? row[k + G] : 0;
     double4 pa = pos[ja], pb = pos[jb];
     {
         const int kn = k + 2 * G;
-        ja = kn < nn ? __ldg(row + kn) : 0;
-        jb = kn + G < nn ? __ldg(row + kn + G) : 0;
+        ja = kn < nn ? row[kn] : 0;
+        jb = kn + G < nn ? row[kn + G] : 0;
     }
     for (; k + G < nn; k += 2 * G) {
         const double4 ca = pa, cb = pb;
         pa = pos[ja];
         pb = pos[jb];
         const int kn = k + 4 * G;
-        ja = kn < nn ? __ldg(row + kn) : 0;
-        jb = kn + G < nn ? __ldg(row + kn + G) : 0;
+        ja = kn < nn ? row[kn] : 0;
+        jb = kn + G < nn ? row[kn + G] : 0;
         double dx, dy, dz;
         sep(ca, dx, dy, dz);
         pair_term<LJ, CO, VIR, SHORT>(c, dx, dy, dz, ca.w, a, near);
@@ -255,16 +258,16 @@ ATVB_DEV void row_mixed(const SysParams& P, const PairSys<float>& S, int s, int 
     bool near;
     int n_near = 0;
     int k = g;
-    int4 pa = pos[k < nn ? __ldg(row + k) : s];
-    int4 pb = pos[k + G < nn ? __ldg(row + k + G) : s];
-    int ia = k + 2 * G < nn ? __ldg(row + k + 2 * G) : s;
-    int ib = k + 3 * G < nn ? __ldg(row + k + 3 * G) : s;
+    int4 pa = pos[k < nn ? row[k] : s];
+    int4 pb = pos[k + G < nn ? row[k + G] : s];
+    int ia = k + 2 * G < nn ? row[k + 2 * G] : s;
+    int ib = k + 3 * G < nn ? row[k + 3 * G] : s;
     for (; k < nn; k += 2 * G) {
         const int4 na = pos[ia];
         const int4 nb = pos[ib];
         const int kn = k + 4 * G;
-        ia = kn < nn ? __ldg(row + kn) : s;
-        ib = kn + G < nn ? __ldg(row + kn + G) : s;
+        ia = kn < nn ? row[kn] : s;
+        ib = kn + G < nn ? row[kn + G] : s;
         float dx, dy, dz;
         sep(pa, dx, dy, dz);
         pair_term<LJ, CO, VIR>(c, dx, dy, dz, __int_as_float(pa.w), a, near);
@@ -381,7 +384,7 @@ ATVB_DEV void fix_share(const SysParams& P, int s, int code, int lane) {
     const int* __restrict__ row = P.nbr + (size_t)s * P.cap;
     const RowConst<float> c = row_const<float>(P, (double)__int_as_float(pi.w));
     for (int k = g + G * lane; k < nn; k += 32 * G) {
-        const int j = __ldg(row + k);
+        const int j = row[k];
         const int4 pj = pos[j];
         const float dx = (float)(int)((unsigned)pi.x - (unsigned)pj.x) * P.Lf_fix[0];
         const float dy = (float)(int)((unsigned)pi.y - (unsigned)pj.y) * P.Lf_fix[1];

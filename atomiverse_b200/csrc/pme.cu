@@ -194,6 +194,12 @@ __global__ void __launch_bounds__(kChunk)
 // the 192^3 mesh at 44 us (FP64) / 28 us (FP32), against 48-77 us / 45-47
 // us when the lanes of an atom split the reads by z offset as the spread
 // does (fewer reads in flight per thread, the splines computed per lane).
+// The mesh is not read through the read-only path (__ldg): as a programmatic
+// dependent this grid is resident while k_fftr_zi writes it.  Plain loads and
+// __ldca are scheduled differently: 21,952 ions, orders 4 / 5 / 6 / 8, FP64
+// 10.7 / 18.4 / 18.3 / 28.8 us plain and 11.6 / 14.9 / 29.2 / 43.9 the other
+// way (registers 126 / 128 / 172 / 234 and 126 / 126 / 128 / 170), mixed
+// 12.4 / 12.6 / 14.5 / 23.0 and 12.4 / 15.3 / 14.4 / 22.9.
 template <bool MIXED, int N>
 __global__ void __launch_bounds__(256)
     k_pme_gather(const Item* items, int nitems, const SysParams* sp) {
@@ -231,7 +237,8 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
                     for (int c = 0; c < N; ++c) {
                         const int g2 = gwrap(b2 + c, K2);
-                        const T cv = __ldg(grid + plane + g2);
+                        const T* at = grid + plane + g2;
+                        const T cv = !MIXED && N == 5 ? __ldca(at) : *at;
                         g0s += cv * dxy * th[2][c];
                         g1s += cv * xdy * th[2][c];
                         g2s += cv * txy * dth[2][c];
