@@ -58,10 +58,12 @@ enum Acc : int {
     kAccCount = 15
 };
 
-// The low words of the pair kernels' sums (SysParams::acc_lo), in units of
-// 2^-31 of the accumulators': LJ, Coulomb, six virials.
-constexpr int kAccLo = 8;
+// The further words of the pair kernels' sums (LJ, Coulomb, six virials) in
+// SysParams::acc_ext: kPairSums low words, in units of 2^-31 of the
+// accumulators', then as many high words, in units of 2^32 of them.
+constexpr int kPairSums = 8;
 constexpr double kAccLoScale = 2147483648.0; // 2^31
+constexpr double kAccHiScale = 4294967296.0; // 2^32
 
 struct SysState {
     unsigned long long acc[kAccCount]; // fixed-point accumulators
@@ -257,7 +259,7 @@ struct SysParams {
     // finished items of k_integrate_a / k_integrate_b: the block that
     // completes the last one runs the system's scalar updates
     unsigned* tickets;
-    unsigned long long* acc_lo; // kAccLo low words of the pair sums
+    unsigned long long* acc_ext; // 2 kPairSums further words of the pair sums
     int *nbr, *nnbr;
     // PME buffers
     unsigned long long* grid_fix;
@@ -291,6 +293,9 @@ ATVB_DEV long long to_fix(double v) { return __double2ll_rn(v * kEFix); }
 ATVB_DEV void red_add_u64(unsigned long long* a, unsigned long long v) {
     asm volatile("red.global.add.u64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
 }
+
+// The accumulator of pair sum k (LJ, Coulomb, six virials).
+ATVB_DEV int pair_acc(int k) { return k == 0 ? kAccELJ : k == 1 ? kAccECoul : kAccVir + k - 2; }
 
 ATVB_DEV void fix_add(unsigned long long* a, double v) {
     red_add_u64(a, (unsigned long long)to_fix(v));

@@ -70,7 +70,7 @@ struct LaunchCfg {
     ItemList pme_real;  // kGridChunk real grid points per item
     const int* sys_list = nullptr; // device list of system indices
     int nsys = 0;
-    int pair_sums = 2;  // energy sums of the pair kernels (kAccLo with a virial)
+    int pair_sums = 2;  // energy sums of the pair kernels (kPairSums with a virial)
     int pair_G = 4;     // lanes per atom of the largest system (reported)
     int any_mixed = 0, any_fp64 = 0;
     int any_snap = 0;   // a system publishes trajectory snapshots

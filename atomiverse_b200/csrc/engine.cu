@@ -643,8 +643,8 @@ Slot::Slot(const atvb_system_desc& d, const DevMem& mem) : desc(d), mem_(mem) {
     hp.small_sort = n <= kSortSmallAtoms ? 1 : 0;
     hp.tickets = (unsigned*)dalloc(2 * sizeof(unsigned));
     CK(cudaMemsetAsync(hp.tickets, 0, 2 * sizeof(unsigned), stream));
-    hp.acc_lo = (unsigned long long*)dalloc(kAccLo * sizeof(unsigned long long));
-    CK(cudaMemsetAsync(hp.acc_lo, 0, kAccLo * sizeof(unsigned long long), stream));
+    hp.acc_ext = (unsigned long long*)dalloc(2 * kPairSums * sizeof(unsigned long long));
+    CK(cudaMemsetAsync(hp.acc_ext, 0, 2 * kPairSums * sizeof(unsigned long long), stream));
     hp.nnbr = di(n);
     hp.cell_count = di(hp.ncell);
     hp.cell_start = di(hp.ncell + 1);
@@ -1049,7 +1049,7 @@ void Engine::build_lists() {
         if (P.prec == kMixed && P.has_lj && !P.general && P.mix_band_lj > 0.0)
             lc_.any_near = 1;
         if (P.need_virial)
-            lc_.pair_sums = kAccLo;
+            lc_.pair_sums = kPairSums;
         if (P.snap_ring)
             lc_.any_snap = 1;
         if (P.baro)
@@ -1893,7 +1893,7 @@ LaunchCfg Engine::restricted_cfg(int id) {
     c.pme_atoms = make_list(list_allocs_, patoms, num_sms_ * 16, mem_);
     c.fft = fft_items(P.has_pme ? std::vector<int>{id} : std::vector<int>{});
     c.any_mixed = P.prec == kMixed;
-    c.pair_sums = P.need_virial ? kAccLo : 2;
+    c.pair_sums = P.need_virial ? kPairSums : 2;
     c.any_fp64 = P.prec != kMixed;
     c.any_near = P.prec == kMixed && P.has_lj && !P.general && P.mix_band_lj > 0.0;
     c.any_baro = P.baro;

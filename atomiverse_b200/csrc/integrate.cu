@@ -206,7 +206,7 @@ __device__ __noinline__ void sys_a_update(const SysParams& P, SysState* st,
 struct ScalarShared {
     SysState st;
     SysParams P;
-    unsigned long long lo[kAccLo];
+    unsigned long long ext[2 * kPairSums];
     int last;
 };
 
@@ -225,8 +225,8 @@ ATVB_DEV void scalar_update(const SysParams& P, ScalarShared& sh, F&& update) {
         l[k] = __ldcg(g + k);
     for (int k = threadIdx.x; k < pwords; k += blockDim.x)
         lp[k] = gp[k];
-    if (threadIdx.x < kAccLo)
-        sh.lo[threadIdx.x] = __ldcg(P.acc_lo + threadIdx.x);
+    if (threadIdx.x < 2 * kPairSums)
+        sh.ext[threadIdx.x] = __ldcg(P.acc_ext + threadIdx.x);
     __syncthreads();
     // an update that may commit a cell writes SysParams itself
     const bool cell = sh.P.thermostat == kNPT || sh.P.baro || sh.P.deform_axis >= 0;
@@ -235,8 +235,8 @@ ATVB_DEV void scalar_update(const SysParams& P, ScalarShared& sh, F&& update) {
     __syncthreads();
     for (int k = threadIdx.x; k < words; k += blockDim.x)
         g[k] = l[k];
-    if (threadIdx.x < kAccLo)
-        P.acc_lo[threadIdx.x] = sh.lo[threadIdx.x];
+    if (threadIdx.x < 2 * kPairSums)
+        P.acc_ext[threadIdx.x] = sh.ext[threadIdx.x];
 }
 
 // The scalar updates of a system by the block that finishes the last of its
@@ -361,26 +361,26 @@ ATVB_DEV double lang_g2pre(const SysParams& P, long long step) {
     return __ddiv_rn(__dsqrt_rn(__ddiv_rn(__dmul_rn(2.0 * kKB, T), P.lang_ddm)), kFtm2v);
 }
 
-// A pair sum of the step: the accumulator, its low word and, for the virial,
-// what the reciprocal sum added; both words are cleared.
-ATVB_DEV double take_sum(SysState* st, int acc, unsigned long long* lo) {
-    const double v =
-        fix_to_d(st->acc[acc]) + (double)(long long)*lo * (kEFixInv / kAccLoScale);
-    st->acc[acc] = 0ull;
-    *lo = 0ull;
+// Pair sum k of the step: the accumulator (for the virial with what the
+// reciprocal sum added to it) and the sum's low and high words; all cleared.
+ATVB_DEV double take_sum(SysState* st, unsigned long long* ext, int k) {
+    unsigned long long *acc = &st->acc[pair_acc(k)], *lo = ext + k, *hi = ext + kPairSums + k;
+    const double v = fix_to_d(*acc) + (double)(long long)*lo * (kEFixInv / kAccLoScale) +
+                     (double)(long long)*hi * (kEFixInv * kAccHiScale);
+    *acc = *lo = *hi = 0ull;
     return v;
 }
 
-// `lo`: the low words of the pair sums (SysParams::acc_lo or a copy of it).
-ATVB_DEV void finish_energy(const SysParams& P, SysState* st, unsigned long long* lo) {
-    st->e_lj = take_sum(st, kAccELJ, lo);
-    st->e_coul = take_sum(st, kAccECoul, lo + 1);
+// `ext`: the further words of the pair sums (SysParams::acc_ext or a copy of it).
+ATVB_DEV void finish_energy(const SysParams& P, SysState* st, unsigned long long* ext) {
+    st->e_lj = take_sum(st, ext, 0);
+    st->e_coul = take_sum(st, ext, 1);
     st->e_recip = fix_to_d(st->acc[kAccERecip]);
     st->acc[kAccERecip] = 0ull;
     st->e_const = P.has_pme ? P.e_const : 0.0;
     st->energy = st->e_lj + st->e_coul + st->e_recip + st->e_const;
     for (int k = 0; k < 6; ++k)
-        st->virial[k] = P.need_virial ? take_sum(st, kAccVir + k, lo + 2 + k)
+        st->virial[k] = P.need_virial ? take_sum(st, ext, 2 + k)
                                       : fix_to_d(st->acc[kAccVir + k]);
     if (P.ext_ev) { // the user components' energy and virial
         st->energy += P.ext_ev[0];
@@ -526,14 +526,14 @@ __global__ void k_baro_scale(const Item* items, int nitems, const SysParams* sp)
 // MTK NPT end of step (nose_hoover_npt.cpp:855-885, P8-P11) from the
 // per-axis kinetic energies of the kicked velocities, then the scalars of
 // the next step's initial half (npt_prepare).
-ATVB_DEV void npt_end_of_step(const SysParams& P, SysState* st, unsigned long long* lo) {
+ATVB_DEV void npt_end_of_step(const SysParams& P, SysState* st, unsigned long long* ext) {
     const double hdt = 0.5 * P.dt;
     double ke[3];
     for (int d = 0; d < 3; ++d) {
         ke[d] = fix_to_d(st->acc[kAccKEX + d]);
         st->acc[kAccKEX + d] = 0ull;
     }
-    finish_energy(P, st, lo); // energies and the virial of this step's forces
+    finish_energy(P, st, ext); // energies and the virial of this step's forces
     st->ke_global = ke[0] + ke[1] + ke[2];
     double s8[3];
     npt_scale_baro(P, st, hdt, ke, s8);                 // P8
@@ -553,9 +553,9 @@ ATVB_DEV void npt_end_of_step(const SysParams& P, SysState* st, unsigned long lo
 // Final-half thermostat, end-of-step scalars, energy history, step counter,
 // on a copy `st` of the system's state.
 __device__ __noinline__ void sys_b_update(const SysParams& P, SysState* st,
-                                          unsigned long long* lo) {
+                                          unsigned long long* ext) {
     if (P.thermostat == kNPT) {
-        npt_end_of_step(P, st, lo);
+        npt_end_of_step(P, st, ext);
         return;
     }
     const double ke = fix_to_d(st->acc[kAccKEB]);
@@ -569,7 +569,7 @@ __device__ __noinline__ void sys_b_update(const SysParams& P, SysState* st,
         st->vscale = 1.0;
         st->kinetic = ke;
     }
-    finish_energy(P, st, lo);
+    finish_energy(P, st, ext);
     st->conserved = st->energy + st->kinetic;
     cell_scalars(P, st);
     if (P.baro)
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kSysThreads)
     }
     scalar_update(P, ss, [&](const SysParams& Q, SysState* st) {
         if (B)
-            sys_b_update(Q, st, ss.lo);
+            sys_b_update(Q, st, ss.ext);
         if (A)
             sys_a_update(Q, st, cond_sort, cond_rows, use_cond);
     });
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(kChunk, 4)
         }
         if (fuse)
             last_item(P, P.tickets + 1, ss,
-                      [&](const SysParams& Q, SysState* st) { sys_b_update(Q, st, ss.lo); });
+                      [&](const SysParams& Q, SysState* st) { sys_b_update(Q, st, ss.ext); });
     }
 }
 
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(kChunk, 3)
             fix_add(&P.st->acc[kAccKEB], 0.5 * kMvv2e * t);
         if (fuse)
             last_item(P, P.tickets, ss, [&](const SysParams& Q, SysState* st) {
-                sys_b_update(Q, st, ss.lo);
+                sys_b_update(Q, st, ss.ext);
                 sys_a_update(Q, st, 0, 0, 0);
             });
     }
@@ -793,7 +793,7 @@ __global__ void k_sys_energy(const int* sys_list, int nsys,
     if (k >= nsys)
         return;
     const SysParams& P = sp[sys_list[k]];
-    finish_energy(P, P.st, P.acc_lo);
+    finish_energy(P, P.st, P.acc_ext);
     P.st->conserved = P.st->energy + P.st->kinetic;
     cell_scalars(P, P.st);
 }
@@ -813,8 +813,8 @@ __global__ void k_force_rebuild(const int* sys_list, int nsys,
     st->acc[kAccELJ] = st->acc[kAccECoul] = st->acc[kAccERecip] = 0ull;
     for (int v = 0; v < 6; ++v)
         st->acc[kAccVir + v] = 0ull;
-    for (int v = 0; v < kAccLo; ++v)
-        sp[sys_list[k]].acc_lo[v] = 0ull;
+    for (int v = 0; v < 2 * kPairSums; ++v)
+        sp[sys_list[k]].acc_ext[v] = 0ull;
     st->nearq_n = 0; // nothing queued by launches outside a force pass counts
     st->nearq_lost = 0;
 }

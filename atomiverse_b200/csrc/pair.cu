@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kPairBlock, MIXED ? 3 : 2)
                     row<false, true, false>(P, S, s, g, G, acc);
             }
         }
-        energy_add(en, acc, S.vir, first);
+        energy_add(en, P, acc, S.vir, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = G / 2; o > 0; o >>= 1) {

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kPairBlock)
             acc.v[k] = 0.0;
         if (s < P.n)
             row_general<MIXED>(P, s, g, acc);
-        energy_add(en, acc, P.need_virial, first);
+        energy_add(en, P, acc, P.need_virial, first);
         double fx = acc.fx, fy = acc.fy, fz = acc.fz;
 #pragma unroll
         for (int o = kGenLanes / 2; o > 0; o >>= 1) {

@@ -233,9 +233,13 @@ ATVB_DEV PairSys<T> pair_sys(const SysParams& P) {
 // depend neither on the order nor on which other systems share the launch;
 // the columns go to the system once per block and system.  (A block sum per
 // item cost two barriers and up to 80 shuffles per 64 atoms.)
-// The columns are dynamic shared memory, `sums` of them (2, or all kAccLo if
-// a system of the launch needs its virial): what they take is L1 the gathers
-// do not have.
+// The columns are dynamic shared memory, `sums` of them (2, or all kPairSums
+// if a system of the launch needs its virial): what they take is L1 the
+// gathers do not have.
+// No word can wrap: a share of 256 eV or more goes to the system straight
+// away, what it has above 2^32 of the accumulator's units in the high word,
+// and a block's sum of 2^18 eV or more is split the same way, so that of
+// 2^12 blocks and 2^32 shares the accumulator receives less than 2^63.
 struct EnergyCols {
     long long* v; // [sum][word][thread]
     int sums;
@@ -243,33 +247,85 @@ struct EnergyCols {
         return v[(2 * k + word) * kPairBlock + threadIdx.x];
     }
 };
+constexpr double kShareFix = 0.5 * kEFix; // 1/2: every pair is visited from both of its atoms
+constexpr int kShareWide = 0x40800000;    // high word of 512.0: a share of 256 eV
+constexpr long long kBlockWide = 1125899906842624; // 2^50
 
 // v into this lane's column of sum k: the first of a system stores.
 ATVB_DEV void energy_add1(const EnergyCols& e, int k, double v, bool first) {
-    const double t = v * (0.5 * kEFix); // 1/2: every pair is visited from both of its atoms
+    const double t = v * kShareFix;
     const long long h = __double2ll_rn(t);
     const long long l = __double2ll_rn((t - (double)h) * kAccLoScale);
     e.at(k, 0) = first ? h : e.at(k, 0) + h;
     e.at(k, 1) = first ? l : e.at(k, 1) + l;
 }
 
-// The row share of every lane of the block (zeros past the last atom).
-// The LJ and Coulomb sums unconditionally: skipping one the system has not
-// made the mixed kernel spill (347 -> 361 us at 262,144 ions).
-ATVB_DEV void energy_add(const EnergyCols& e, const PairAcc& a, bool vir, bool first) {
-    energy_add1(e, 0, a.elj, first);
-    energy_add1(e, 1, a.ec, first);
-    if (vir && e.sums == kAccLo)
+ATVB_DEV int share_size(double v) { return __double2hiint(v) & 0x7fffffff; }
+
+// A share v of sum k that energy_add1 has added, if it is wide (256 eV or more
+// in size, or not a number: atoms that nearly coincide): out of the column
+// again and straight to the system.  Shares are cut off where the sum of as
+// many as the system can have would leave the high word (2^37 eV in a million
+// atoms); not a number counts as the largest.
+ATVB_DEV void energy_wide1(const EnergyCols& e, const SysParams& P, int k, double v) {
+    if (share_size(v) < kShareWide)
+        return;
+    const double t = v * kShareFix;
+    const long long h0 = __double2ll_rn(t);
+    e.at(k, 0) -= h0;
+    e.at(k, 1) -= __double2ll_rn((t - (double)h0) * kAccLoScale);
+    const double most = 4611686018427387904.0 / (32.0 * P.n); // 2^62 / shares
+    double a = fmin(fabs(t) * (1.0 / kAccHiScale), most);
+    a = t < 0.0 ? -a : a;
+    const double hi = floor(a);
+    const double r = (a - hi) * kAccHiScale; // exact
+    const long long h = __double2ll_rn(r);
+    const long long l = __double2ll_rn((r - (double)h) * kAccLoScale);
+    red_add_u64(&P.st->acc[pair_acc(k)], (unsigned long long)h);
+    red_add_u64(P.acc_ext + k, (unsigned long long)l);
+    red_add_u64(P.acc_ext + kPairSums + k, (unsigned long long)(long long)hi);
+}
+
+static __device__ __noinline__ void energy_wide(EnergyCols e, const SysParams& P, bool vir,
+                                                double elj, double ec, double v0, double v1,
+                                                double v2, double v3, double v4, double v5) {
+    energy_wide1(e, P, 0, elj);
+    energy_wide1(e, P, 1, ec);
+    if (vir) {
+        const double v[6] = {v0, v1, v2, v3, v4, v5};
 #pragma unroll
         for (int k = 0; k < 6; ++k)
+            energy_wide1(e, P, 2 + k, v[k]);
+    }
+}
+
+// The row share of every lane of the block (zeros past the last atom).
+// The LJ and Coulomb sums unconditionally: skipping one the system has not
+// made the mixed kernel spill (347 -> 361 us at 262,144 ions).  One test for
+// wide shares, after the columns (1,000,188 LJ atoms with virial 408 us a
+// launch without it, 408 with, 423 with a test before each column; 108,000 of
+// a mixture 92, 95 and 98, mixed 61.8, 63.9 and 66.0).
+ATVB_DEV void energy_add(const EnergyCols& e, const SysParams& P, const PairAcc& a, bool vir,
+                         bool first) {
+    vir = vir && e.sums == kPairSums;
+    int size = max(share_size(a.elj), share_size(a.ec));
+    energy_add1(e, 0, a.elj, first);
+    energy_add1(e, 1, a.ec, first);
+    if (vir)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            size = max(size, share_size(a.v[k]));
             energy_add1(e, 2 + k, a.v[k], first);
+        }
+    if (size >= kShareWide)
+        energy_wide(e, P, vir, a.elj, a.ec, a.v[0], a.v[1], a.v[2], a.v[3], a.v[4], a.v[5]);
 }
 
 // Block-uniform.  `again`: the block goes on to another system.
 ATVB_DEV void energy_flush(const EnergyCols& e, const SysParams& P, bool again) {
     __syncthreads();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    static_assert(kPairBlock / 32 >= kAccLo, "a warp per sum");
+    static_assert(kPairBlock / 32 >= kPairSums, "a warp per sum");
     if (w < (P.need_virial ? e.sums : 2)) {
         long long h = 0, l = 0;
 #pragma unroll
@@ -279,12 +335,15 @@ ATVB_DEV void energy_flush(const EnergyCols& e, const SysParams& P, bool again) 
         }
         h = warp_sum(h);
         l = warp_sum(l);
-        const int acc = w == 0 ? kAccELJ : w == 1 ? kAccECoul : kAccVir + w - 2;
         if (lane == 0) {
+            if (h >= kBlockWide || h <= -kBlockWide) {
+                red_add_u64(P.acc_ext + kPairSums + w, (unsigned long long)(h >> 32));
+                h &= 0xffffffffll;
+            }
             if (h)
-                red_add_u64(&P.st->acc[acc], (unsigned long long)h);
+                red_add_u64(&P.st->acc[pair_acc(w)], (unsigned long long)h);
             if (l)
-                red_add_u64(&P.acc_lo[w], (unsigned long long)l);
+                red_add_u64(P.acc_ext + w, (unsigned long long)l);
         }
     }
     if (again)
