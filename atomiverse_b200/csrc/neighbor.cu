@@ -400,8 +400,9 @@ ATVB_DEV unsigned special_class(const SysParams& P, int i, int j) {
 // further apart than half an edge.  Its error is bounded (apply_box): below
 // fband_lo a candidate is certainly listed, at or above fband_hi certainly
 // not.  A candidate in between is appended, and a row that got one is
-// settled once it is complete (settle_row) by the exact FP64 test, so the
-// listed set is exactly the FP64 one.
+// settled once it is complete (settle_row; exact_rows if it has outgrown its
+// places) by the exact FP64 test, so the listed set and its length are exactly
+// the FP64 ones.
 //
 // Bound by instruction issue (63 % of the issue slots at 24 warps per SM).
 // What a window costs before its first atom (finding each lane's column,
@@ -435,15 +436,69 @@ ATVB_DEV float3 frame_pos(const SysParams& P, int4 q, int4 org) {
                        (float)(int)((unsigned)q.z - (unsigned)org.z) * P.Lf_fix[2]);
 }
 
-// The entries of atom i's row (cnt of them, those below the capacity stored)
-// whose FP32 distance is in the error band, decided by the exact FP64 test:
-// the row is compacted in place, in order.  About one row in a thousand.
-// Returns the new length.  (A row cut at its capacity keeps the entries it
-// has; it is reported and rebuilt.)
+// Row i has its final length: more than its places is reported.
+ATVB_DEV void row_done(const SysParams& P, int i, int len) {
+    P.nnbr[i] = min(len, P.cap);
+    if (len > P.cap) {
+        // the row is cut: pairs are missing until rows are widened
+        atomicOr(&P.st->overflow, 1);
+        atomicOr(&P.st->status, kStatusRowOverflow);
+    }
+}
+
+// The rows of cell c among those of atoms [cs, ce) that build_share left open
+// (length -1): they have candidates of the error band and, with them, more
+// entries than places, so which of those not stored are pairs could not be
+// told afterwards, nor whether the row fits.  Built from the start in the same
+// order, every candidate decided by the exact FP64 test before it is counted.
+// A call inside build_share costs it registers: cell sort and build of a
+// million atoms 146.0 us a step without these rows, 147.5 with them, 148.9
+// with the call inside (262,144 ions 131.3, 131.8, 133.1).
+__device__ __noinline__ void exact_rows(const SysParams& P, int c, int cs, int ce, int* s_max,
+                                        unsigned* s_sum) {
+    const int lane = threadIdx.x & 31;
+    const double L[3] = {P.L[0], P.L[1], P.L[2]};
+    const double hL[3] = {P.halfL[0], P.halfL[1], P.halfL[2]};
+    const double rl2 = P.rlist2;
+    const int nc0 = P.nc[0], nc1 = P.nc[1], nc2 = P.nc[2];
+    const int cz = c % nc2, cy = (c / nc2) % nc1, cx = c / (nc1 * nc2);
+    for (int i = cs; i < ce; ++i) {
+        if (P.nnbr[i] >= 0)
+            continue; // warp-uniform
+        int* row = P.nbr + (size_t)i * P.cap;
+        const double4 a = P.posd4[i];
+        int len = 0;
+        __syncwarp();
+        for (int col = 0; col < P.ncol; ++col) {
+            int a0, l0, a1, l1;
+            column_runs(nc0, nc1, nc2, P.cell_start, P.cols[col], cx, cy, cz, a0, l0, a1, l1);
+            for (int t0 = 0; t0 < l0 + l1; t0 += 32) {
+                const int t = t0 + lane;
+                const int j = t < l0 ? a0 + t : a1 + t - l0;
+                const bool hit =
+                    t < l0 + l1 && j != i && exact_r2(a, P.posd4[j], L, hL) < rl2;
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                const int w = len + __popc(m & ((1u << lane) - 1u));
+                if (hit && w < P.cap)
+                    row[w] = (int)((unsigned)j |
+                                   (P.has_special ? special_class(P, i, j) << 30 : 0u));
+                len += __popc(m);
+            }
+        }
+        if (lane == 0) {
+            row_done(P, i, len);
+            atomicMax(s_max, len);
+            atomicAdd(s_sum, (unsigned)len);
+        }
+    }
+}
+
+// The entries of atom i's row (cnt of them, all stored) whose FP32 distance is
+// in the error band, decided by the exact FP64 test: the row is compacted in
+// place, in order.  About one row in a thousand.  Returns the new length.
 __device__ __noinline__ int settle_row(const SysParams& P, int i, int org_i, int cnt) {
     const int lane = threadIdx.x & 31;
     int* row = P.nbr + (size_t)i * P.cap;
-    const int stored = min(cnt, P.cap);
     const double L[3] = {P.L[0], P.L[1], P.L[2]};
     const double hL[3] = {P.halfL[0], P.halfL[1], P.halfL[2]};
     const float Lx = (float)L[0], Ly = (float)L[1], Lz = (float)L[2];
@@ -453,10 +508,10 @@ __device__ __noinline__ int settle_row(const SysParams& P, int i, int org_i, int
     const float3 a = frame_pos(P, P.lpos[i], org);
     int out = 0;
     __syncwarp();
-    for (int k0 = 0; k0 < stored; k0 += 32) {
+    for (int k0 = 0; k0 < cnt; k0 += 32) {
         const int k = k0 + lane;
         int e = 0;
-        bool keep = k < stored;
+        bool keep = k < cnt;
         if (keep) {
             e = row[k];
             const int j = e & (int)kRowIdxMask;
@@ -473,13 +528,13 @@ __device__ __noinline__ int settle_row(const SysParams& P, int i, int org_i, int
         out += __popc(m);
         __syncwarp();
     }
-    return cnt - stored + out;
+    return out;
 }
 
 template <bool FOLD, bool SP>
 ATVB_DEV void build_share(const SysParams& P, int c, int cs, int ce, int lane,
                           float4* __restrict__ sr, int4* __restrict__ sc, int* s_max,
-                          unsigned* s_sum) {
+                          unsigned* s_sum, int* s_open) {
     const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
     // every field the loops use, read once: the row stores below could alias
     // SysParams as far as the compiler knows
@@ -588,25 +643,25 @@ ATVB_DEV void build_share(const SysParams& P, int c, int cs, int ce, int lane,
             if (a >= ni)
                 break;
             int len = (int)(off[a] - a * cap);
-            if (amb & (1u << a))
-                len = settle_row(P, i0 + a, cs, len);
+            if (amb & (1u << a)) {
+                if (len <= (int)cap) {
+                    len = settle_row(P, i0 + a, cs, len);
+                } else { // left to exact_rows
+                    len = -1;
+                    *s_open = 1;
+                }
+            }
             if (lane == a)
                 cnt = len;
         }
         const int wmax = __reduce_max_sync(full, cnt);
-        const int wsum = __reduce_add_sync(full, cnt);
+        const int wsum = __reduce_add_sync(full, max(cnt, 0));
         if (lane == 0) {
             atomicMax(s_max, wmax);
             atomicAdd(s_sum, (unsigned)wsum);
         }
-        if (lane < ni) {
-            P.nnbr[i0 + lane] = min(cnt, (int)cap);
-            if (cnt > (int)cap) {
-                // the row is cut: pairs are missing until rows are widened
-                atomicOr(&P.st->overflow, 1);
-                atomicOr(&P.st->status, kStatusRowOverflow);
-            }
-        }
+        if (lane < ni)
+            row_done(P, i0 + lane, cnt);
     }
 }
 
@@ -621,6 +676,7 @@ __global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
     // 0.5 ms of the build of 1,000,188 LJ atoms)
     __shared__ int s_max;
     __shared__ unsigned s_sum;
+    __shared__ int s_open[kListWarps]; // the warp's share has rows for exact_rows
     int cur = -1;
     auto flush = [&] { // block-uniform
         __syncthreads();
@@ -659,19 +715,29 @@ __global__ void __launch_bounds__(32 * kListWarps, kListBlocks)
         const int ce = c_lo + ((c_n * (part + 1)) >> split_log2);
         if (cs >= ce)
             continue;
+        if (lane == 0)
+            s_open[warp] = 0;
+        __syncwarp();
         if (P.lframe_ok) {
             if (P.has_special)
-                build_share<false, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum);
+                build_share<false, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum,
+                                         &s_open[warp]);
             else
                 build_share<false, false>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max,
-                                          &s_sum);
+                                          &s_sum, &s_open[warp]);
         } else {
             if (P.has_special)
-                build_share<true, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum);
+                build_share<true, true>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max, &s_sum,
+                                        &s_open[warp]);
             else
                 build_share<true, false>(P, c, cs, ce, lane, sr[warp], sc[warp], &s_max,
-                                         &s_sum);
+                                         &s_sum, &s_open[warp]);
         }
+        __syncwarp();
+        const bool open = s_open[warp] != 0;
+        __syncwarp();
+        if (open)
+            exact_rows(P, c, cs, ce, &s_max, &s_sum);
     }
     if (cur >= 0)
         flush();
