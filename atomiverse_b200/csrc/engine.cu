@@ -2172,6 +2172,7 @@ void Engine::set_lj_types(int id, int ncoef, const int32_t* ti, const int32_t* t
     sl->lj_tj.assign(tj, tj + ncoef);
     sl->lj_eps.assign(eps, eps + ncoef);
     sl->lj_sig.assign(sigma, sigma + ncoef);
+    sl->table_types.clear(); // a table built by an upload that then failed is void
     sl->ntypes = nt;
     sl->hp.general = 1;
     push_params(id);
@@ -2270,6 +2271,7 @@ void Engine::set_special_bonds(int id, const double lj[3], const double coul[3],
     sl->bond_a.assign(a, a + nbonds);
     sl->bond_b.assign(b, b + nbonds);
     sl->special_set = true;
+    sl->special_tags.clear(); // as for the LJ table
     sl->hp.general = 1;
     push_params(id);
     dirty_ = true;

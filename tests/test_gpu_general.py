@@ -182,6 +182,31 @@ def test_configuration_after_upload_is_refused(atvb, ctx):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [0, 1])
+def test_coefficients_changed_after_a_failed_upload(atvb, ctx, precision):
+    # an upload refused for its bonds has already made the LJ table; the next
+    # one, with other coefficients and sound bonds, must not keep it
+    desc, frame, coeffs, special = _water(m=7)
+    desc = dict(desc, precision=precision, nl_cutoff=8.0, lj_cutoff=8.0, coul_cutoff=8.0)
+    bad = dict(special, bonds=list(special["bonds"]) + [(1, 10 ** 9)])
+    s = atvb.System(ctx, desc, None, lj_types=[(0, 0, 0.02, 2.5)], special_bonds=bad)
+    with pytest.raises(atvb.AtvbError):
+        s.upload(frame)
+    args, keep = atvb._lj_type_args(coeffs)
+    atvb.check(s.lib.atvb_system_set_lj_types(s._h, *args))
+    args, keep = atvb._special_args(special)
+    atvb.check(s.lib.atvb_system_set_special_bonds(s._h, *args))
+    s.upload(frame)
+    fresh = atvb.System(ctx, desc, frame, lj_types=coeffs, special_bonds=special)
+    for x in (s, fresh):
+        x.compute_forces()
+    (fa, sa), (fb, sb) = s.download(), fresh.download()
+    for k in fa:
+        assert np.array_equal(fa[k], fb[k]), k
+    assert sa["energy"] == sb["energy"] and sa["energy_lj"] == sb["energy_lj"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
 def test_cpp_water_matches_python(atvb, ctx, tmp_path, precision):
     """md::MD with per-type PairLJCut, special bonds and PME (C++ mirror)
     gives bit for bit what the Python layer gives for the same frame."""
