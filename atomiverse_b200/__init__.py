@@ -94,6 +94,12 @@ def _soa(frame: dict, n: int, writable: bool = False) -> tuple[SoaView, list]:
     return v, keep
 
 
+def _outputs(keys, n: int) -> dict:
+    """Arrays for a frame to be read into: those the library fills need no
+    initial value, any other key stays zero."""
+    return {k: np.empty(n) if k in FRAME_KEYS else np.zeros(n) for k in keys}
+
+
 def _lj_type_args(coeffs):
     """ctypes arguments for (type_i, type_j, epsilon, sigma) coefficients."""
     ti = np.array([c[0] for c in coeffs], dtype=np.int32)
@@ -280,7 +286,7 @@ class System:
         """Frame and scalars.  A sticky status bit (wrong or non-finite
         physics in some step) raises PhysicsError unless check=False; its
         `result` carries the (frame, scalars) anyway."""
-        out = {k: np.empty(self.n) for k in keys}
+        out = _outputs(keys, self.n)
         v, keep = _soa(out, self.n, writable=True)
         s = Scalars()
         rc = self.lib.atvb_system_download(self._h, C.byref(v), C.byref(s))
@@ -425,7 +431,7 @@ class Batch:
         check(self.lib.atvb_batch_step(self._h, int(n)))
 
     def download(self, k: int, keys=FRAME_KEYS, check: bool = True) -> tuple[dict, dict]:
-        out = {key: np.empty(self.sizes[k]) for key in keys}
+        out = _outputs(keys, self.sizes[k])
         v, keep = _soa(out, self.sizes[k], writable=True)
         s = Scalars()
         rc = self.lib.atvb_batch_download(self._h, int(k), C.byref(v), C.byref(s))
@@ -508,7 +514,7 @@ class Server:
 
     def collect(self, rid: int) -> tuple[dict, dict]:
         n = self.sizes[rid]
-        out = {k: np.empty(n) for k in FRAME_KEYS[:9]}
+        out = _outputs(FRAME_KEYS[:9], n)
         v, keep = _soa(out, n, writable=True)
         r = _abi.RequestResult()
         check(self.lib.atvb_server_collect(self._h, int(rid), C.byref(v), C.byref(r)))

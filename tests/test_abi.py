@@ -101,3 +101,31 @@ int main() {
                                 os.path.join(ROOT, "include"), os.path.join(cpp, name)],
                                capture_output=True, text=True)
             assert r.returncode == 0, (name, r.stderr)
+
+
+def test_download_fills_every_array_it_returns(atvb, monkeypatch):
+    """Keys a download does not fill come back as zeros, not as whatever the
+    heap held (the library's part played by a stub)."""
+    import numpy as np
+    monkeypatch.setattr(atvb.np, "empty", lambda n: np.full(n, np.nan))
+
+    class Lib:
+        def atvb_system_download(self, h, view, scalars):
+            v = view._obj
+            for k in atvb.FRAME_KEYS:
+                p = getattr(v, k)
+                if p:
+                    for i in range(5):
+                        p[i] = 1.0
+            return 0
+
+        atvb_batch_download = lambda self, h, k, view, s: self.atvb_system_download(h, view, s)
+
+    s, b = atvb.System.__new__(atvb.System), atvb.Batch.__new__(atvb.Batch)
+    s._h = b._h = None
+    s.lib = b.lib = Lib()
+    s.n, b.sizes = 5, [5]
+    keys = ("x", "vz", "charge", "tag", "type", "nonsense")
+    for out, _ in (s.download(keys), b.download(0, keys)):
+        for k in keys:
+            assert np.array_equal(out[k], np.full(5, float(k in atvb.FRAME_KEYS))), k
