@@ -108,8 +108,9 @@ struct Xfer {
     size_t bytes;
 };
 
-// Pinned staging between pageable host arrays and the device: kPiece bytes,
-// two per worker, allocated on the first large call and kept by the engine.
+// Copies between host arrays and the device; pageable ones from kStagedFrom
+// bytes a call through pinned buffers of kPiece bytes, two per worker,
+// allocated on the first such call and kept by the engine.
 class HostStage {
   public:
     explicit HostStage(int device) : device_(device) {}
@@ -124,6 +125,7 @@ class HostStage {
     static constexpr size_t kStagedFrom = size_t(8) << 20; // bytes of a call
     static constexpr int kMaxWorkers = 4;
     void ready();
+    void move(const std::vector<Xfer>& list, cudaStream_t stream, bool out);
     void run(const std::vector<Xfer>& list, cudaStream_t stream, bool out);
     int device_;
     int workers_ = 1;

@@ -10,6 +10,8 @@
   (cpu/frame/pbc.h:48-50), so the forces are those of the wrapped frame;
 - neutral ions beside charged ones with real-space Ewald and PME (real-space
   terms with q == 0 skipped, coul_long.cpp:146-222) and a net charge;
+- frames of several megabytes in pageable and pinned arrays, all of one kind
+  or mixed, come back as they went up;
 - an empty system is refused when it is created, and a system or batch with
   nothing uploaded refuses to step, each with an error the caller can read.
 """
@@ -173,3 +175,34 @@ def test_empty_and_unuploaded_systems_are_refused(atvb, ctx):
     with pytest.raises(atvb.AtvbError, match="upload"):
         b.step(1)
     b.close()
+
+
+@pytest.mark.parametrize("pinned", ["none", "all", "positions", "all but positions"])
+def test_large_frames_in_pageable_and_pinned_arrays(atvb, ctx, pinned):
+    import ctypes as C
+
+    import torch
+    rng = np.random.default_rng(5)
+    m = 62
+    n = m ** 3  # 1.9 MB an array: staged from five pageable ones on
+    g = (np.arange(m) + 0.5) * 1.1
+    pos = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    pos += rng.uniform(-0.1, 0.1, size=pos.shape)
+    frame = dict(x=pos[:, 0], y=pos[:, 1], z=pos[:, 2],
+                 **{k: rng.normal(size=n) for k in ("vx", "vy", "vz", "fx", "fy", "fz", "charge")},
+                 mass=rng.uniform(1.0, 2.0, size=n))
+
+    def is_pinned(k):
+        return pinned == "all" or (pinned != "none" and (k in "xyz") == (pinned == "positions"))
+
+    def array(k, v):
+        v = np.ascontiguousarray(v, dtype=np.float64)
+        return torch.from_numpy(v).pin_memory().numpy() if is_pinned(k) else v.copy()
+
+    up = {k: array(k, v) for k, v in frame.items()}
+    s = atvb.System(ctx, _lj_desc(n, (m * 1.1,) * 3), up)
+    down = {k: array(k, np.full(n, np.nan)) for k in frame}
+    view, keep = atvb._soa(down, n, writable=True)
+    atvb.check(s.lib.atvb_system_download(s._h, C.byref(view), None))
+    for k, v in frame.items():
+        assert np.array_equal(down[k], v), k
