@@ -41,6 +41,28 @@ def test_long_calls_equal_single_steps(atvb, ctx, precision, thermostat, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("thermostat", [0, 1, 2])
+def test_a_first_long_call_runs_the_longer_graph(atvb, ctx, thermostat):
+    from atomiverse_b200 import workloads as W
+    desc, frame = W.lj_fcc(ncell=6, seed=4, thermostat=thermostat)
+    desc.update(tau=50.0)
+    one, many, short = (atvb.System(ctx, desc, frame) for _ in range(3))
+    for s in (one, many, short):
+        s.compute_forces()
+    for _ in range(70):
+        one.step(1)
+    per_step = one.launch_count()
+    many.step(70)
+    # 8 launches of eight steps, a pass less between two steps of each where
+    # no sum of the whole system stands between the halves
+    merged = 0 if thermostat == 1 else 8 * 7
+    assert many.launch_count() == 70 * per_step - merged
+    short.step(20)  # too short to pay for the capture
+    assert short.launch_count() == 20 * per_step
+    _same(one.download(), many.download())
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("precision", [0, 1])
 def test_uneven_batch_equals_single_steps(atvb, ctx, precision):
     from atomiverse_b200 import workloads as W
