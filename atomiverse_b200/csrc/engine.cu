@@ -227,20 +227,28 @@ static int expected_row(const atvb_system_desc& d, const Geometry& g) {
     return std::min(cap, std::max(nmax, 32));
 }
 
+// Device bytes of a system as its Slot allocates them, rows at their first
+// capacity.
 size_t estimate_bytes(const atvb_system_desc& d) {
     Geometry g = make_geometry(d);
     const size_t n = (size_t)d.n_atoms;
     const int cap = expected_row(d, g);
-    size_t b = n * (14 * 8 + 8 + 32 + 32 + 6 * 4 + (size_t)cap * 4);
-    if (d.precision == ATVB_MIXED)
-        b += n * 16;
-    b += (size_t)(g.nc[0] * g.nc[1] * g.nc[2] + 1) * 8;
-    b += sizeof(SysState) + 3 * 8 * 4096;
+    const bool mixed = d.precision == ATVB_MIXED;
+    // 14 double arrays and the tags; posd4, f4, lpos, pos4; perm, rank,
+    // cell_of, slot, nnbr and perm0; the rows
+    size_t b = n * (14 * 8 + 8 + 32 + 32 + 16 + (mixed ? 16 : 32) + 5 * 4 + 8 + (size_t)cap * 4);
+    if (mixed && d.lj_enabled)
+        b += std::max<size_t>(4096, n / 16) * 8;
+    const size_t ncell = (size_t)g.nc[0] * g.nc[1] * g.nc[2];
+    b += (2 * ncell + 1 + (ncell + kScanChunk - 1) / kScanChunk) * 4 + g.cols.size() * 16;
+    const size_t hist = d.history_capacity > 0 ? d.history_capacity : 4096;
+    b += sizeof(SysState) + (2 * kPairSums + 1) * 8 + 3 * 8 * hist;
     if (d.pme_enabled) {
         const size_t K0 = pme_K(d, g, 0), K1 = pme_K(d, g, 1),
                      K2 = pme_K(d, g, 2);
         const size_t nt = K0 * K1 * K2, nh = K0 * K1 * ((K2 / 2 + 1 + 15) / 16 * 16);
-        const size_t rs = d.precision == ATVB_MIXED ? 4 : 8;
+        const size_t rs = mixed ? 4 : 8;
+        b += n * 32; // fp4
         b += nt * 8 + nt * rs + nh * 2 * rs + (K0 + K1 + K2) * 8;
         b += (K0 + K1 + K2) * 2 * rs; // roots of unity of the transforms
     }

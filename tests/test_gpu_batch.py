@@ -185,6 +185,31 @@ def test_served_arrivals_while_running_equal_alone(atvb, ctx):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision,pme", [(0, False), (1, False), (0, True), (1, True)])
+def test_request_bytes_is_what_a_system_takes(atvb, ctx, precision, pme):
+    # short rows, so that what an atom takes beside its row weighs; large
+    # enough that the pool's 32 MB blocks do not
+    import torch
+    m = 150 if not pme else 120
+    n, L = m ** 3, 4.0 * m
+    desc = dict(n_atoms=n, box=(L, L, L), precision=precision, nl_cutoff=5.0, nl_skin=0.5,
+                lj_enabled=1, lj_epsilon=1e-3, lj_sigma=3.0, lj_cutoff=5.0, dt=1.0)
+    if pme:
+        desc.update(coul_enabled=1, coul_alpha=0.4, coul_cutoff=5.0, pme_enabled=1,
+                    pme_alpha=0.4, pme_order=4, pme_grid=(64, 64, 64))
+    g = (np.arange(m) + 0.5) * 4.0
+    pos = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    frame = dict(x=pos[:, 0].copy(), y=pos[:, 1].copy(), z=pos[:, 2].copy(), mass=np.ones(n))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info(0)[0]
+    s = atvb.System(ctx, desc, frame)
+    took = before - torch.cuda.mem_get_info(0)[0]
+    s.close()
+    want = atvb.request_bytes(desc)
+    assert abs(took / want - 1.0) < 0.03
+
+
+@pytest.mark.gpu
 def test_server_admission_cancel_and_errors(atvb, ctx):
     from atomiverse_b200 import workloads as W
     d1, f1 = W.lj_fcc(ncell=5, seed=21, precision=1)
