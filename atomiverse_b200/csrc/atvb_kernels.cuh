@@ -13,7 +13,7 @@ constexpr long long kCondMinAtoms = 100000; // engines from this size skip them 
                                             // conditional graph nodes
 constexpr int kListChunk = 4;   // warp tasks per item of the list build
 constexpr int kScanChunk = 2048; // cells per item of the cell scan
-constexpr int kSortSmallAtoms = 65536; // largest system whose cell sort runs in one
+constexpr int kSortSmallAtoms = 49152; // largest system whose cell sort runs in one
                                        // cluster (k_sort_small)
 constexpr int kGridChunk = 4096; // grid points per item of the PME grid kernels
 constexpr int kLaneClasses = 6;  // pair lanes per atom: 1, 2, 4, 8, 16, 32

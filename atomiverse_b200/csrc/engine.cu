@@ -1320,12 +1320,12 @@ void Engine::enqueue_step_components() {
     ++comp_step_;
 }
 
-// Kernel launches of one step.
 // Launches of one list build: the cell sorts and the rows.
 int64_t Engine::rebuild_kernels() const {
     return (lc_.nsmall ? 1 : 0) + (lc_.sort_atoms.n ? 5 : 0) + 1;
 }
 
+// Kernel launches of one step.
 int64_t Engine::kernels_per_step() const {
     int64_t k = 0;
     k += 1;                                   // integrate_a

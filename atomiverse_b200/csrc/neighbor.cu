@@ -220,9 +220,10 @@ __global__ void k_permute(const Item* items, int nitems, const SysParams* sp) {
 // cluster of eight blocks, with cluster barriers between the stages: one
 // launch instead of five on every step of an engine too small for the
 // conditional build nodes (about 1 us each on the steps without a build).
-// Per pass against one block up to 8,192 atoms and five kernels above: 4,000
-// atoms 2.48 -> 2.38 ms, 13,500 2.38 -> 2.20, 14,039 2.17 -> 2.00, 22,176
-// ions 4.64 -> 4.46; 256 atoms 1.91 -> 1.95 (the cluster's launch).
+// Step of an LJ system with one build in seven, five kernels / one cluster:
+// 256 atoms 23.7 / 19.6 us, 4,000 28.1 / 23.6, 8,192 31.2 / 26.0, 16,384 35.8
+// / 32.3, 32,768 48.8 / 47.3, 49,152 56.4 / 56.6, 65,536 67.2 / 68.2, 98,000
+// 87.1 / 93.0: the line is where they meet (eight SMs build for the rest).
 // Data of other blocks of the cluster is read past L1 (__ldcg).
 constexpr int kSortThreads = 1024, kSortCtas = 8;
 

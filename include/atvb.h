@@ -186,7 +186,11 @@ int atvb_system_compute_forces(atvb_system* sys);
 int atvb_system_step(atvb_system* sys, int32_t n_steps);
 /* atvb_system_step with a CUDA event on the system's stream before the
  * first step and after every step; step_ms (n_steps entries, may be NULL)
- * gets each step's device time, *total_ms the whole span.  Synchronises. */
+ * gets each step's device time, *total_ms the whole span.  Synchronises.
+ * Every step is a launch of its own: a long atvb_system_step runs eight steps
+ * per launch, with the final half of a step and the initial half of the next
+ * in one kernel for NVE and Langevin, and takes a few microseconds a step
+ * less than the times given here. */
 int atvb_system_step_timed(atvb_system* sys, int32_t n_steps, double* step_ms,
                            double* total_ms);
 int atvb_system_download(atvb_system* sys, atvb_soa_view* frame,
@@ -387,11 +391,12 @@ int atvb_system_profile_read(atvb_system* sys, atvb_kernel_time* out,
 /* Lanes per atom in the pair kernel (1,2,4,8,16,32); 0 = autotune. */
 int atvb_system_set_pair_lanes(atvb_system* sys, int32_t lanes);
 /* Kernel launches of the last step() call, counting the list-build kernels on
- * every step (six; two if every system has at most 65,536 atoms, seven if
+ * every step (six; two if every system has at most 49,152 atoms, seven if
  * systems on both sides of that share an engine): in the step graph of a
  * system (or batch) of at least 100,000 atoms they launch only on steps
  * where a system rebuilds its list (conditional nodes), so the launches made
- * there are this count less that many per step without a rebuild. */
+ * there are this count less that many per step without a rebuild.  Launches
+ * that a long call saves between its steps are not counted. */
 int atvb_system_launch_count(atvb_system* sys, int64_t* launches);
 /* The system's CUDA stream (cudaStream_t) for event timing by callers. */
 void* atvb_system_stream(atvb_system* sys);

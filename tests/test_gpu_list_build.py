@@ -48,8 +48,9 @@ def test_pairs_at_the_edge_of_the_list(atvb, ctx, orc, cells, jitter):
     (3000, (9.0, 9.5, 10.0), 4.0),    # dense cells, several warps and passes per cell
     (900, (30.0, 31.0, 33.0), 1.2),   # sparse, reach 1
     (8193, (21.0, 22.0, 23.0), 2.2),  # long cells; more atoms than the sort's threads
-    (65536, (40.0, 41.0, 43.0), 0.9),  # the largest sort in one cluster
-    (65537, (40.0, 41.0, 43.0), 0.9),  # and the smallest in several kernels
+    (49152, (40.0, 41.0, 43.0), 0.9),  # the largest sort in one cluster
+    (49153, (40.0, 41.0, 43.0), 0.9),  # and the smallest in several kernels
+    (65537, (40.0, 41.0, 43.0), 0.9),
     (20000, (20.48, 20.48, 81.92), 1.0),  # several scan chunks
 ])
 def test_random_positions(atvb, ctx, orc, n, box, rc):
