@@ -267,14 +267,15 @@ ATVB_DEV int share_size(double v) { return __double2hiint(v) & 0x7fffffff; }
 // again and straight to the system.  Shares are cut off where the sum of as
 // many as the system can have would leave the high word (2^37 eV in a million
 // atoms); not a number counts as the largest.
-ATVB_DEV void energy_wide1(const EnergyCols& e, const SysParams& P, int k, double v) {
+ATVB_DEV void energy_wide(const EnergyCols& e, const SysParams& P, int k, double v) {
     if (share_size(v) < kShareWide)
         return;
     const double t = v * kShareFix;
     const long long h0 = __double2ll_rn(t);
     e.at(k, 0) -= h0;
     e.at(k, 1) -= __double2ll_rn((t - (double)h0) * kAccLoScale);
-    const double most = 4611686018427387904.0 / (32.0 * P.n); // 2^62 / shares
+    // 2^57 over the next power of two of the atoms (32 shares each): no division
+    const double most = __hiloint2double((1023 + 57 - (32 - __clz(P.n))) << 20, 0);
     double a = fmin(fabs(t) * (1.0 / kAccHiScale), most);
     a = t < 0.0 ? -a : a;
     const double hi = floor(a);
@@ -286,25 +287,14 @@ ATVB_DEV void energy_wide1(const EnergyCols& e, const SysParams& P, int k, doubl
     red_add_u64(P.acc_ext + kPairSums + k, (unsigned long long)(long long)hi);
 }
 
-static __device__ __noinline__ void energy_wide(EnergyCols e, const SysParams& P, bool vir,
-                                                double elj, double ec, double v0, double v1,
-                                                double v2, double v3, double v4, double v5) {
-    energy_wide1(e, P, 0, elj);
-    energy_wide1(e, P, 1, ec);
-    if (vir) {
-        const double v[6] = {v0, v1, v2, v3, v4, v5};
-#pragma unroll
-        for (int k = 0; k < 6; ++k)
-            energy_wide1(e, P, 2 + k, v[k]);
-    }
-}
-
 // The row share of every lane of the block (zeros past the last atom).
 // The LJ and Coulomb sums unconditionally: skipping one the system has not
 // made the mixed kernel spill (347 -> 361 us at 262,144 ions).  One test for
-// wide shares, after the columns (1,000,188 LJ atoms with virial 408 us a
-// launch without it, 408 with, 423 with a test before each column; 108,000 of
-// a mixture 92, 95 and 98, mixed 61.8, 63.9 and 66.0).
+// wide shares, after the columns, and no call behind it (a division is one,
+// too): 1,000,188 LJ atoms with virial 408 us a launch without it, 406 so, 423
+// with a test before each column and a call; 108,000 atoms of a mixture 92.0,
+// 92.2 and 98; steps of 13,500 of them 45.3, 45.6 and, with one test and a
+// call, 48.6 us.
 ATVB_DEV void energy_add(const EnergyCols& e, const SysParams& P, const PairAcc& a, bool vir,
                          bool first) {
     vir = vir && e.sums == kPairSums;
@@ -317,8 +307,14 @@ ATVB_DEV void energy_add(const EnergyCols& e, const SysParams& P, const PairAcc&
             size = max(size, share_size(a.v[k]));
             energy_add1(e, 2 + k, a.v[k], first);
         }
-    if (size >= kShareWide)
-        energy_wide(e, P, vir, a.elj, a.ec, a.v[0], a.v[1], a.v[2], a.v[3], a.v[4], a.v[5]);
+    if (size >= kShareWide) {
+        energy_wide(e, P, 0, a.elj);
+        energy_wide(e, P, 1, a.ec);
+        if (vir)
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                energy_wide(e, P, 2 + k, a.v[k]);
+    }
 }
 
 // Block-uniform.  `again`: the block goes on to another system.
