@@ -189,6 +189,8 @@ def test_served_arrivals_while_running_equal_alone(atvb, ctx):
 def test_request_bytes_is_what_a_system_takes(atvb, ctx, precision, pme):
     # short rows, so that what an atom takes beside its row weighs; large
     # enough that the pool's 32 MB blocks do not
+    import gc
+
     import torch
     m = 150 if not pme else 120
     n, L = m ** 3, 4.0 * m
@@ -200,6 +202,7 @@ def test_request_bytes_is_what_a_system_takes(atvb, ctx, precision, pme):
     g = (np.arange(m) + 0.5) * 4.0
     pos = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
     frame = dict(x=pos[:, 0].copy(), y=pos[:, 1].copy(), z=pos[:, 2].copy(), mass=np.ones(n))
+    gc.collect()  # systems of earlier tests give their memory back before, not meanwhile
     torch.cuda.synchronize()
     before = torch.cuda.mem_get_info(0)[0]
     s = atvb.System(ctx, desc, frame)
